@@ -16,7 +16,7 @@ OK, BAD_ARGS, TOO_LARGE, CODEGEN_FAIL, CHIP_FAIL, NAN_WEIGHT = 0, -1, -2, -3, -4
 ENGINE_AUTO, ENGINE_FMA, ENGINE_MMA = 0, 1, 2
 
 if not os.path.exists(LIB_PATH):
-    raise ImportError("libb200moe.so is not built: run `python -m cudapp_b200.build` (needs nvcc); no CPU fallback exists")
+    raise ImportError("libb200moe.so is not built: run `python cudapp_b200/build.py` (needs nvcc); no CPU fallback exists")
 lib = C.CDLL(LIB_PATH)
 
 

@@ -1,6 +1,6 @@
 """Builds libb200moe.so (the C-ABI product library) in-tree with nvcc for sm_100a.
 
-    python -m cudapp_b200.build [--force]
+    python cudapp_b200/build.py [--force]      (the package itself cannot be imported before its library exists)
 
 Sources: cudapp_b200/csrc/*.cu; output: cudapp_b200/lib/libb200moe.so. Objects are rebuilt when a source or
 header is newer than them. No torch, no JIT cache: the shared object travels with the tree.

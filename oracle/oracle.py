@@ -23,7 +23,7 @@ def build(ref=False):
     """Compile the checker (and, with ref=True and the reference tree present, the reference build)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
     where = os.environ.get("B200MOE_REFERENCE", os.path.normpath(os.path.join(HERE, "..", "..", "reference")))   # beside this repository's folder
-    if ref and os.path.isdir(where):
+    if ref and os.path.exists(os.path.join(where, "src", "omega_gpu_fp8_pack.c")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + where], check=True)
 
 
