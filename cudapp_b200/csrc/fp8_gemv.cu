@@ -7,11 +7,10 @@
 // step; lanes are summed by a shuffle-down tree 16, 8, 4, 2, 1. The reference folds 2^-120 / 2^64 / 2^56 into
 // w / x / scale because its integer byte decode yields e4m3 * 2^-120; here cvt.f16x2.e4m3x2 decodes exactly, so
 // no fold is stored (the folds are exact powers of two whose product is 1: same bits).
-//
-// Weight bytes are streamed once with 16/8/4-byte loads per lane (512/256/128 contiguous bytes per warp) and
-// decoded in registers; R output rows per warp share each x chunk, MT activation rows share each weight chunk.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <stdlib.h>
+#include <vector>
 #include "internal.h"
 
 namespace b200 {
@@ -27,32 +26,26 @@ __device__ __forceinline__ void decode4(uint32_t v, float *o) {
     const float2 f0 = __half22float2(*reinterpret_cast<__half2 *>(&lo)), f1 = __half22float2(*reinterpret_cast<__half2 *>(&hi));
     o[0] = f0.x; o[1] = f0.y; o[2] = f1.x; o[3] = f1.y;
 }
-template <int LB> __device__ __forceinline__ void load_w(const uint8_t *p, float *o) {
-    typename WVec<LB>::T v = __ldcs(reinterpret_cast<const typename WVec<LB>::T *>(p));  // streaming: read once
-    const uint32_t *u = reinterpret_cast<const uint32_t *>(&v);
-#pragma unroll
-    for (int i = 0; i < LB / 4; i++) decode4(u[i], o + 4 * i);
-}
-template <int LB> __device__ __forceinline__ void load_x(const void *x, int bf16, uint32_t c0, float *o) {
-    if (bf16) {
-        const uint16_t *p = reinterpret_cast<const uint16_t *>(x) + c0;
-#pragma unroll
-        for (int i = 0; i < LB / 4; i++) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p) + i);
-            o[4 * i] = __uint_as_float(v.x << 16); o[4 * i + 1] = __uint_as_float(v.x & 0xffff0000u);
-            o[4 * i + 2] = __uint_as_float(v.y << 16); o[4 * i + 3] = __uint_as_float(v.y & 0xffff0000u);
-        }
-    } else {
-        const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + c0);
-#pragma unroll
-        for (int i = 0; i < LB / 4; i++) { const float4 v = __ldg(p + i); o[4 * i] = v.x; o[4 * i + 1] = v.y; o[4 * i + 2] = v.z; o[4 * i + 3] = v.w; }
-    }
-}
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+// (q-th float4 of a lane's LB columns): the xor spreads the four float4 of neighbouring lanes over all banks when a row is written to shared memory
+template <int LB> __device__ __forceinline__ uint32_t xs_at(uint32_t q, uint32_t lane) { return q * 32u + (lane ^ (q * (LB == 16 ? 2u : LB == 8 ? 4u : 0u))); }
 
-// grid (ctas, groups or segments); block 256 (8 warps). Warp task: R consecutive output rows x one pass of MT activation rows.
+// grid (ctas, groups or segments); 4 warps. A CTA puts MT activation rows of its segment into shared memory as f32, in the lanes' own column
+// order, and its warps then stream weight rows against them: R consecutive output rows per warp, the weights of the next two K steps in flight.
+// Bound by HBM when a segment has a few rows (64 tokens x 8 picks, [1536, 2048]: 400 MB), by the FP32 pipe from about four rows per expert on.
+// With one output row per warp and x read per row from global memory, as this kernel was, every product cost a load and a conversion beside its
+// FMA; four rows share them here, and fma.rn.f32x2 runs two rows' chains (each its own IEEE chain: the same bits) in one instruction slot.
+constexpr uint32_t ROWS_WARPS = 4;
+template <int MT> constexpr uint32_t ROWS_CHUNK = MT == 8 ? 2048u : 4096u;   // columns of x resident at a time: at most 64 KB, so that three CTAs share an SM
 template <int LB, int R, int MT>
-__global__ void __launch_bounds__(256) fp8_rows_kernel(const GemvArgs a) {
-    const uint32_t g = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+__global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? 5 : 3) fp8_rows_kernel(const __grid_constant__ GemvArgs a) {
+    constexpr uint32_t STEP = 32u * LB, CS = ROWS_CHUNK<MT> / STEP, Q = LB / 4, NT = 32u * ROWS_WARPS;
+    constexpr int PF = R == 1 ? 4 : 2, PAIRS = R > 1 ? R / 2 : 1;
+    using WT = typename WVec<LB>::T;
+    extern __shared__ float4 xs[];                 // [step of the chunk][MT][Q][32]
+    __shared__ const uint8_t *s_row[MT];
+    const uint32_t g = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint64_t w_va, s_va; uint32_t row0, cnt;
     if (a.seg) {
         const Seg32 sg = a.seg[g];
@@ -60,103 +53,168 @@ __global__ void __launch_bounds__(256) fp8_rows_kernel(const GemvArgs a) {
         if (cnt == 0) return;
     } else {
         const uint32_t gg = (a.mutant == 3 && (g ^ 1u) < a.groups_or_segs) ? (g ^ 1u) : g;
-        w_va = a.tab[2 * gg]; s_va = a.tab[2 * gg + 1]; row0 = g; cnt = 1;
+        w_va = a.tab ? a.tab[2 * gg] : a.tab_inline[2 * gg]; s_va = a.tab ? a.tab[2 * gg + 1] : a.tab_inline[2 * gg + 1]; row0 = g; cnt = 1;
     }
-    const uint8_t *W = reinterpret_cast<const uint8_t *>(w_va);
-    const float *S = reinterpret_cast<const float *>(s_va);
-    const uint32_t n = a.n, k = a.k, kb = k / 128u, steps = k / (32u * LB);
+    const uint32_t n = a.n, k = a.k, kb = k / 128u, steps = k / STEP;
     const size_t xstride = a.x_stride_bytes ? a.x_stride_bytes : (size_t)k * (a.x_bf16 ? 2 : 4);
-    for (uint32_t rb = (blockIdx.x * nw + warp) * R; rb < n; rb += gridDim.x * nw * R) {
-        const uint8_t *wrow = W + (size_t)rb * k + lane * LB;
-        const float *srow = S + (size_t)(rb / 128u) * kb;   // R divides 128: the R rows share a scale row
-        for (uint32_t i0 = 0; i0 < cnt; i0 += MT) {
-            float acc[R][MT];
-            const uint8_t *xr[MT];
-#pragma unroll
-            for (int m = 0; m < MT; m++) {
-                uint32_t p = row0 + (i0 + m < cnt ? i0 + m : i0);
-                if (a.seg && a.mutant == 3 && (p ^ 1u) < a.rows) p ^= 1u;
-                const uint32_t xi = a.seg ? (a.xmap ? a.xmap[p] : p) : (a.x_rows == 1 ? 0u : p);
-                xr[m] = reinterpret_cast<const uint8_t *>(a.x) + (size_t)xi * xstride;
-#pragma unroll
-                for (int j = 0; j < R; j++) acc[j][m] = 0.0f;
-            }
-#pragma unroll(R == 1 && MT == 1 ? 4 : 2)   // one row per warp: all four 16-byte weight loads of a 2048-wide row in flight
-            for (uint32_t st = 0; st < steps; st++) {
-                const uint32_t c0 = st * 32u * LB + lane * LB;
-                float wv[R][LB];
-#pragma unroll
-                for (int j = 0; j < R; j++) load_w<LB>(wrow + (size_t)j * k + (size_t)st * 32u * LB, wv[j]);
-                const float sc = a.mutant == 1 ? 1.0f : __ldg(srow + (a.mutant == 2 ? 0u : c0 / 128u));
+    for (uint32_t i0 = 0; i0 < cnt; i0 += MT) {
+        const uint32_t mc = min((uint32_t)MT, cnt - i0);
+        if (i0) __syncthreads();                   // the previous pass has read its rows
+        if (tid < mc) {
+            uint32_t p = row0 + i0 + tid;
+            if (a.seg && a.mutant == 3 && (p ^ 1u) < a.rows) p ^= 1u;
+            const uint32_t xi = a.seg ? (a.xmap ? a.xmap[p] : p) : (a.x_rows == 1 ? 0u : p);
+            s_row[tid] = reinterpret_cast<const uint8_t *>(a.x) + (size_t)xi * xstride;
+        }
+        __syncthreads();
+        auto stage = [&](uint32_t first) {         // columns [first, first + chunk) of the pass's rows
+            const uint32_t cols = min(ROWS_CHUNK<MT>, k - first);
+            for (uint32_t c = tid * 4u; c < cols; c += NT * 4u) {
+                float4 v[MT];
 #pragma unroll
                 for (int m = 0; m < MT; m++) {
-                    float xv[LB];
-                    load_x<LB>(xr[m], a.x_bf16, c0, xv);
+                    v[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if ((uint32_t)m >= mc) continue;
+                    if (a.x_bf16) {
+                        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(s_row[m] + (size_t)(first + c) * 2));
+                        v[m] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+                    } else v[m] = __ldg(reinterpret_cast<const float4 *>(s_row[m] + (size_t)(first + c) * 4));
+                }
+                const uint32_t st = c / STEP, rem = c % STEP;
+                float4 *to = xs + (size_t)st * MT * Q * 32u + xs_at<LB>((rem % LB) / 4u, rem / LB);
+#pragma unroll
+                for (int m = 0; m < MT; m++) if ((uint32_t)m < ((mc + 1u) & ~1u) || MT == 1) to[m * Q * 32] = v[m];
+            }
+            __syncthreads();
+        };
+        const bool resident = k <= ROWS_CHUNK<MT>;
+        WT raw[PF][R]; float sc[PF];
+        auto fetch = [&](int slot, uint32_t rb, uint32_t st) {
+            const uint8_t *wrow = reinterpret_cast<const uint8_t *>(w_va) + (size_t)rb * k + lane * LB;
+            const float *srow = reinterpret_cast<const float *>(s_va) + (size_t)(rb / 128u) * kb;   // R divides 128: the R rows share a scale row
+#pragma unroll
+            for (int j = 0; j < R; j++) raw[slot][j] = __ldcs(reinterpret_cast<const WT *>(wrow + (size_t)j * k + (size_t)st * STEP));   // streaming: read once
+            sc[slot] = a.mutant == 1 ? 1.0f : __ldg(srow + (a.mutant == 2 ? 0u : (st * STEP + lane * LB) / 128u));
+        };
+        const uint32_t rb0 = (blockIdx.x * ROWS_WARPS + warp) * R;
+#pragma unroll
+        for (int i = 0; i < PF; i++) if ((uint32_t)i < steps && rb0 < n) fetch(i, rb0, i);   // on its way while x is staged
+        if (resident) stage(0);
+        for (uint32_t rb = rb0; rb < n; rb += gridDim.x * ROWS_WARPS * R) {   // n is a multiple of 4 R: every warp makes the same number of turns
+            uint64_t acc[MT][PAIRS];               // R > 1: two rows each; R = 1: the low half
+#pragma unroll
+            for (int m = 0; m < MT; m++)
+#pragma unroll
+                for (int p = 0; p < PAIRS; p++) acc[m][p] = 0;
+            for (uint32_t st0 = 0; st0 < steps; st0 += PF) {
+#pragma unroll
+                for (int i = 0; i < PF; i++) {
+                    const uint32_t st = st0 + i;
+                    if (st >= steps) break;
+                    if (!resident && st % CS == 0) { if (st || rb >= gridDim.x * ROWS_WARPS * R) __syncthreads(); stage(st * STEP); }
+                    float wv[R][LB];
 #pragma unroll
                     for (int j = 0; j < R; j++) {
-                        float dot = 0.0f;
+                        const uint32_t *u = reinterpret_cast<const uint32_t *>(&raw[i][j]);
 #pragma unroll
-                        for (int b = 0; b < LB; b++) dot = fmaf(wv[j][b], xv[b], dot);
-                        acc[j][m] = fmaf(dot, sc, acc[j][m]);
+                        for (int b = 0; b < LB / 4; b++) decode4(u[b], wv[j] + 4 * b);
+                    }
+                    const float s = sc[i];
+                    // this slot's next weights: of this row group, or the first ones of the group after it
+                    const bool more = st + PF < steps;
+                    const uint32_t nrb = more ? rb : rb + gridDim.x * ROWS_WARPS * R;
+                    if (nrb < n) fetch(i, nrb, more ? st + PF : (uint32_t)i);
+                    const float4 *xst = xs + (size_t)(st % CS) * MT * Q * 32u;
+#pragma unroll
+                    for (int m0 = 0; m0 < MT; m0 += 2) {
+                        if ((uint32_t)m0 >= mc) break;
+#pragma unroll
+                        for (int m = m0; m < (m0 + 2 < MT ? m0 + 2 : MT); m++) {
+                            float xv[LB];
+#pragma unroll
+                            for (int q = 0; q < (int)Q; q++) *reinterpret_cast<float4 *>(xv + 4 * q) = xst[m * Q * 32 + xs_at<LB>(q, lane)];
+                            if constexpr (R > 1) {
+#pragma unroll
+                                for (int p = 0; p < PAIRS; p++) {
+                                    uint64_t dot = 0;
+#pragma unroll
+                                    for (int b = 0; b < LB; b++) dot = fma2(pack2(wv[2 * p][b], wv[2 * p + 1][b]), pack2(xv[b], xv[b]), dot);
+                                    acc[m][p] = fma2(dot, pack2(s, s), acc[m][p]);
+                                }
+                            } else {
+                                float dot = 0.0f;
+#pragma unroll
+                                for (int b = 0; b < LB; b++) dot = fmaf(wv[0][b], xv[b], dot);
+                                acc[m][0] = pack2(fmaf(dot, s, __uint_as_float((uint32_t)acc[m][0])), 0.0f);
+                            }
+                        }
                     }
                 }
             }
 #pragma unroll
-            for (int j = 0; j < R; j++)
+            for (int m = 0; m < MT; m++) {
+                if ((uint32_t)m >= mc) break;
+                float v[R];
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    float v = acc[j][m];
-#pragma unroll
-                    for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                    if (lane == 0 && i0 + m < cnt) {
-                        const uint32_t p = row0 + i0 + m;
-                        const uint32_t yi = (a.seg && a.ymap) ? a.ymap[p] : p;
-                        a.y[(size_t)yi * n + rb + j] = v * a.out_mul;
-                    }
+                for (int p = 0; p < PAIRS; p++) { v[R > 1 ? 2 * p : 0] = __uint_as_float((uint32_t)acc[m][p]); if (R > 1) v[R > 1 ? 2 * p + 1 : 0] = __uint_as_float((uint32_t)(acc[m][p] >> 32)); }
+                // the shuffle-down tree's lane-0 sum: an exchange adds the same pairs (addition commutes), and with four rows the first two exchanges also
+                // deal the rows to the lane quarters, so the tree costs 6 shuffles instead of 20 and the four results leave as one 16-byte run
+                float t; uint32_t j = 0; bool out = lane == 0;
+                if constexpr (R == 4) {
+                    const bool h16 = lane & 16u, h8 = lane & 8u;
+                    const float a0 = (h16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16), a1 = (h16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+                    t = (h8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h8 ? a0 : a1, 8);
+                    j = (h16 ? 2u : 0u) + (h8 ? 1u : 0u); out = (lane & 7u) == 0;
+                } else {
+                    t = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+                    t += __shfl_xor_sync(0xffffffffu, t, 8);
                 }
+                t += __shfl_xor_sync(0xffffffffu, t, 4); t += __shfl_xor_sync(0xffffffffu, t, 2); t += __shfl_xor_sync(0xffffffffu, t, 1);
+                if (out) {
+                    const uint32_t p = row0 + i0 + m, yi = (a.seg && a.ymap) ? a.ymap[p] : p;
+                    a.y[(size_t)yi * n + rb + j] = t * a.out_mul;
+                }
+            }
         }
     }
 }
 
+template <int LB, int R, int MT>
+static cudaError_t launch_one(const GemvArgs &a, dim3 grid, cudaStream_t s) {
+    const size_t smem = (size_t)MT * (a.k < ROWS_CHUNK<MT> ? a.k : ROWS_CHUNK<MT>) * 4;
+    static const cudaError_t attr = cudaFuncSetAttribute(fp8_rows_kernel<LB, R, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MT * ROWS_CHUNK<MT> * 4));
+    if (attr != cudaSuccess) return attr;
+    fp8_rows_kernel<LB, R, MT><<<grid, 32 * ROWS_WARPS, smem, s>>>(a);
+    return cudaGetLastError();
+}
 template <int R, int MT>
 static cudaError_t launch_lb(const GemvArgs &a, dim3 grid, cudaStream_t s) {
     const uint32_t k = a.k;
-    if (k % 512u == 0) fp8_rows_kernel<16, R, MT><<<grid, 256, 0, s>>>(a);
-    else if (k % 256u == 0) fp8_rows_kernel<8, R, MT><<<grid, 256, 0, s>>>(a);
-    else fp8_rows_kernel<4, R, MT><<<grid, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    if (k % 512u == 0) return launch_one<16, R, MT>(a, grid, s);
+    if (k % 256u == 0) return launch_one<8, R, MT>(a, grid, s);
+    return launch_one<4, R, MT>(a, grid, s);
 }
 
-// GEMV forms: one activation row per group. CTAs per group chosen to put about four 8-warp CTAs on every SM.
+// GEMV forms: one activation row per group. Four rows per warp once that leaves every SM two CTAs; below it one row per warp gives four times the
+// CTAs. A row's arithmetic does not depend on how rows are dealt to warps: same bits.
 cudaError_t launch_gemv_grouped(const GemvArgs &a, uint32_t cta_budget, uint32_t *grid_x, uint32_t *warps, cudaStream_t s) {
     const uint32_t sms = st().sm_count ? st().sm_count : 148u;
-    const uint32_t row_groups = a.n / 4u;                    // R = 4 rows per warp task
-    uint32_t gx = (row_groups + 7u) / 8u;                    // one task per warp
-    uint32_t want = cta_budget ? cta_budget : (sms * 4u + a.groups_or_segs - 1u) / a.groups_or_segs;
-    if (want == 0) want = 1;
-    if (gx > want) gx = want;
-    if (warps) *warps = 8;
-    if (gx * a.groups_or_segs < sms && !cta_budget) {
-        // few groups (the single-projection call): four rows per warp would leave most SMs without a CTA; one row per warp gives
-        // four times the CTAs. A row's arithmetic does not depend on how rows are dealt to warps: same bits.
-        gx = (a.n + 7u) / 8u;
-        if (gx > want) gx = want;
-        if (grid_x) *grid_x = gx;
-        return launch_lb<1, 1>(a, dim3(gx, a.groups_or_segs), s);
-    }
+    const bool few = (uint64_t)(a.n / 16u) * a.groups_or_segs < 2u * sms && !cta_budget;
+    uint32_t gx = few ? a.n / ROWS_WARPS : a.n / (4u * ROWS_WARPS);
+    if (cta_budget && gx > cta_budget) gx = cta_budget;
+    if (warps) *warps = ROWS_WARPS;
     if (grid_x) *grid_x = gx;
-    return launch_lb<4, 1>(a, dim3(gx, a.groups_or_segs), s);
+    return few ? launch_lb<1, 1>(a, dim3(gx, a.groups_or_segs), s) : launch_lb<4, 1>(a, dim3(gx, a.groups_or_segs), s);
 }
-// Row-table form: MT = 4 activation rows per pass of a segment's weights.
+static uint32_t gemm_rows_mt(uint32_t k) { return k <= ROWS_CHUNK<8> ? 8u : 4u; }
+// Row-table form: up to eight activation rows per pass of a segment's weights (four where eight rows of x would leave room for one CTA per SM).
+// A CTA keeps its rows of x for several 16-row weight groups: about twelve CTAs per SM in all (three at a time), so that long and short segments even out.
 cudaError_t launch_gemm_rows(const GemvArgs &a, uint32_t *grid_x, uint32_t *mt, cudaStream_t s) {
-    const uint32_t sms = st().sm_count ? st().sm_count : 148u;
-    uint32_t gx = (a.n + 7u) / 8u;
-    uint32_t want = (sms * 4u + a.groups_or_segs - 1u) / a.groups_or_segs;
-    if (want == 0) want = 1;
-    if (gx > want) gx = want;
+    const uint32_t sms = st().sm_count ? st().sm_count : 148u, groups = a.n / (4u * ROWS_WARPS), want = (sms * 12u + a.groups_or_segs - 1u) / a.groups_or_segs;
+    const uint32_t per = (groups + want - 1u) / want, gx = (groups + per - 1u) / per, rows = gemm_rows_mt(a.k);
     if (grid_x) *grid_x = gx;
-    if (mt) *mt = 4;
-    return launch_lb<1, 4>(a, dim3(gx, a.groups_or_segs), s);
+    if (mt) *mt = rows;
+    return rows == 8u ? launch_lb<4, 8>(a, dim3(gx, a.groups_or_segs), s) : launch_lb<4, 4>(a, dim3(gx, a.groups_or_segs), s);
 }
 
 // ---------------------------------------------------------------- host-staged API cores
@@ -174,6 +232,60 @@ static void fill_info(OmegaGpuFp8Info *info, const OmegaGpuFp8Tensor *t, uint32_
     info->general = lb == 4u || groups > OMEGA_GPU_FP8_MAX_GROUPS;
 }
 
+// whether a result still holds the poison it was filled with: sets a flag in mapped host memory
+__global__ void __launch_bounds__(256) poison_scan_kernel(const float4 *__restrict__ y, size_t n4, uint32_t *flag) {
+    bool bad = false;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
+        const float4 v = __ldg(y + i);
+        bad |= v.x == POISON_F32 || v.y == POISON_F32 || v.z == POISON_F32 || v.w == POISON_F32;
+    }
+    if (bad) *flag = 1;
+}
+
+// A host call's result. Up to RESULT_BYTES the kernel stores it straight into mapped host memory, which was filled with poison before the launch: the
+// host takes each word as soon as it is no longer poison, and the call pays neither a fill kernel nor a copy nor a stream synchronisation (a single
+// [768, 2048] projection: 49 -> about 12 us per call). Larger results are poisoned, scanned and copied from device memory.
+struct HostResult {
+    float *dev = nullptr; volatile float *mapped = nullptr; void *area = nullptr; size_t count; cudaStream_t s;
+    bool open(size_t words, cudaStream_t stream) {
+        count = words; s = stream; area = result_area();
+        if (!area) return false;
+        if (words * 4 <= RESULT_BYTES) {
+            mapped = (volatile float *)area;
+            for (size_t i = 0; i < words; i++) mapped[i] = POISON_F32;
+            dev = (float *)area;   // unified addressing: the host's pointer is the device's
+            return true;
+        }
+        dev = (float *)stage(2, words * 4);
+        if (dev) launch_fill_f32(dev, words, POISON_F32, s);
+        return dev != nullptr;
+    }
+    // 0, or CHIP_FAIL with the error text set; y is written only when every word was produced. sync: the caller reads events afterwards
+    int take(float *y, bool sync, const char *what) {
+        bool left = false;
+        if (mapped) {
+            if (!sync) {   // bounded: past the limit the stream decides (a fault, a result word that equals the poison)
+                const uint64_t until = now_ns() + 2000000;
+                for (size_t i = 0; i < count; i++)
+                    for (uint32_t spin = 1; mapped[i] == POISON_F32; spin++)
+                        if (spin % 1024 == 0 && now_ns() > until) { sync = true; i = count - 1; break; }
+            }
+            if (sync && !cuda_ok(cudaStreamSynchronize(s), what)) return OMEGA_GPU_FP8_CHIP_FAIL;
+            if (sync) for (size_t i = 0; i < count; i++) left |= mapped[i] == POISON_F32;
+            if (!left) memcpy(y, area, count * 4);
+        } else {
+            volatile uint32_t *flag = result_flag(area);
+            *flag = 0;
+            const size_t blocks = (count / 4 + 255) / 256;
+            poison_scan_kernel<<<(unsigned)(blocks < 592 ? blocks : 592), 256, 0, s>>>((const float4 *)dev, count / 4, (uint32_t *)flag);   // count: rows of a multiple of 128 values
+            if (!cuda_ok(cudaGetLastError(), "poison scan launch") || !to_host(y, dev, count * 4, s, flag) || !cuda_ok(cudaStreamSynchronize(s), what)) return OMEGA_GPU_FP8_CHIP_FAIL;
+            left = *flag != 0;
+        }
+        if (left) { set_error("output poison survived"); return OMEGA_GPU_FP8_CHIP_FAIL; }
+        return OMEGA_GPU_FP8_OK;
+    }
+};
+
 // ids / x on the host, or tab / x on the device (dev form). y always a host buffer here.
 static int gemv_core(const OmegaGpuFp8Tensor *t, uint32_t groups, const uint32_t *ids, const float *x32, const uint16_t *x16,
                      uint32_t x_rows, float *y, OmegaGpuFp8Info *info, uint64_t dev_tab, uint64_t dev_x) {
@@ -186,43 +298,34 @@ static int gemv_core(const OmegaGpuFp8Tensor *t, uint32_t groups, const uint32_t
     State &g = st();
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
     const uint32_t n = t->n, k = t->k;
-    const size_t xbytes = (size_t)x_rows * k * (x16 ? 2 : 4), ybytes = (size_t)groups * n * 4;
-    uint64_t *tab = (uint64_t *)stage(0, (size_t)groups * 16);
-    void *xd = stage(1, xbytes); float *yd = (float *)stage(2, ybytes);
-    if (!tab || !xd || !yd) return OMEGA_GPU_FP8_CHIP_FAIL;
     cudaStream_t s = g.stream;
-    bool ok = true;
-    if (!dev_tab) {
-        uint64_t *ht = (uint64_t *)malloc((size_t)groups * 16);
-        if (!ht) return OMEGA_GPU_FP8_BAD_ARGS;
-        for (uint32_t i = 0; i < groups; i++) (void)omega_gpu_fp8_tensor_entry(t, ids[i], &ht[2 * i], &ht[2 * i + 1]);
-        ok = cuda_ok(cudaMemcpyAsync(tab, ht, (size_t)groups * 16, cudaMemcpyHostToDevice, s), "copy group table") && cuda_ok(cudaStreamSynchronize(s), "copy group table");
-        free(ht);
-    }
-    if (ok && !dev_x) ok = cuda_ok(cudaMemcpyAsync(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, cudaMemcpyHostToDevice, s), "copy x");
-    if (!ok) return OMEGA_GPU_FP8_CHIP_FAIL;
-    launch_fill_f32(yd, (size_t)groups * n, POISON_F32, s);
     GemvArgs a = {};
-    a.tab = dev_tab ? (const uint64_t *)(uintptr_t)dev_tab : tab;
-    a.x = dev_x ? (const void *)(uintptr_t)dev_x : xd; a.x_bf16 = (!dev_x && x16) ? 1 : 0; a.x_rows = x_rows;
-    a.y = yd; a.n = n; a.k = k; a.groups_or_segs = groups; a.rows = groups;
+    if (dev_tab) a.tab = (const uint64_t *)(uintptr_t)dev_tab;
+    else if (groups <= sizeof a.tab_inline / 16) for (uint32_t i = 0; i < groups; i++) (void)omega_gpu_fp8_tensor_entry(t, ids[i], &a.tab_inline[2 * i], &a.tab_inline[2 * i + 1]);
+    else {
+        std::vector<uint64_t> ht((size_t)groups * 2);
+        for (uint32_t i = 0; i < groups; i++) (void)omega_gpu_fp8_tensor_entry(t, ids[i], &ht[2 * i], &ht[2 * i + 1]);
+        uint64_t *tab = (uint64_t *)stage(0, ht.size() * 8);
+        if (!tab || !to_device(tab, ht.data(), ht.size() * 8, s)) return OMEGA_GPU_FP8_CHIP_FAIL;
+        a.tab = tab;
+    }
+    if (!dev_x) {
+        const size_t xbytes = (size_t)x_rows * k * (x16 ? 2 : 4);
+        void *xd = stage(1, xbytes);
+        if (!xd || !to_device(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, s)) return OMEGA_GPU_FP8_CHIP_FAIL;
+        a.x = xd;
+    } else a.x = (const void *)(uintptr_t)dev_x;
+    HostResult r;
+    if (!r.open((size_t)groups * n, s)) return OMEGA_GPU_FP8_CHIP_FAIL;
+    a.x_bf16 = (!dev_x && x16) ? 1 : 0; a.x_rows = x_rows;
+    a.y = r.dev; a.n = n; a.k = k; a.groups_or_segs = groups; a.rows = groups;
     a.out_mul = dev_x ? 5.421010862427522e-20f /* 2^-64: the reference router's fold on x' */ : 1.0f;
     a.mutant = g.gemv_mutant;
     uint32_t gx = 0, warps = 0;
-    cudaEventRecord(g.ev0, s);
-    ok = cuda_ok(launch_gemv_grouped(a, g.cta_budget, &gx, &warps, s), "gemv launch");
-    cudaEventRecord(g.ev1, s);
-    float *yh = (float *)malloc(ybytes);
-    if (!yh) return OMEGA_GPU_FP8_BAD_ARGS;
-    ok = ok && cuda_ok(cudaMemcpyAsync(yh, yd, ybytes, cudaMemcpyDeviceToHost, s), "copy y") && cuda_ok(cudaStreamSynchronize(s), "gemv");
-    int rc = ok ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;
-    if (ok) {
-        size_t unchanged = 0;
-        for (size_t i = 0; i < (size_t)groups * n; i++) if (yh[i] == POISON_F32) unchanged++;
-        if (unchanged) { set_error("output poison survived"); rc = OMEGA_GPU_FP8_CHIP_FAIL; }
-        else memcpy(y, yh, ybytes);
-    }
-    free(yh);
+    if (info) cudaEventRecord(g.ev0, s);
+    bool ok = cuda_ok(launch_gemv_grouped(a, g.cta_budget, &gx, &warps, s), "gemv launch");
+    if (info) cudaEventRecord(g.ev1, s);
+    const int rc = ok ? r.take(y, info != nullptr, "gemv") : OMEGA_GPU_FP8_CHIP_FAIL;
     fill_info(info, t, groups, gx, warps);
     if (info && ok) { float ms = 0; if (cudaEventElapsedTime(&ms, g.ev0, g.ev1) == cudaSuccess) info->elapsed_ns = (uint64_t)(ms * 1e6); info->completion_marker = 1; }
     if (info) info->call_ns = now_ns() - t0;
@@ -243,52 +346,38 @@ static int gemm_core(const OmegaGpuFp8Tensor *t, uint32_t M, const uint32_t *ids
     State &g = st();
     if (!dev_open()) return OMEGA_GPU_FP8GEMM_CHIP_FAIL;
     const uint32_t n = t->n, k = t->k;
-    const size_t xbytes = (size_t)x_rows * k * (x16 ? 2 : 4), ybytes = (size_t)M * n * 4;
-    Seg32 *hseg = (Seg32 *)calloc(segs, sizeof(Seg32));
-    if (!hseg) return OMEGA_GPU_FP8GEMM_BAD_ARGS;
-    uint32_t sg = 0, passes_max = 0; uint64_t streamed = 0;
+    const size_t xbytes = (size_t)x_rows * k * (x16 ? 2 : 4), sbytes = (size_t)segs * sizeof(Seg32);
+    std::vector<uint8_t> tables(sbytes + (size_t)M * 4);   // segment records, then the row table: one copy
+    Seg32 *hseg = (Seg32 *)tables.data();
+    memcpy(tables.data() + sbytes, trow, (size_t)M * 4);
+    uint32_t sg = 0; uint64_t passes = 0, passes_max = 0;
+    const uint32_t mt = gemm_rows_mt(k);
     for (uint32_t i = 0; i < M;) {
         uint32_t j = i; while (j < M && ids[j] == ids[i]) j++;
         (void)omega_gpu_fp8_tensor_entry(t, ids[i], &hseg[sg].w_va, &hseg[sg].s_va);
         hseg[sg].row0 = i; hseg[sg].cnt = j - i;
-        const uint32_t passes = (j - i + 3u) / 4u; if (passes > passes_max) passes_max = passes;
-        streamed += (uint64_t)passes * n * k;
+        const uint32_t p = (j - i + mt - 1u) / mt; if (p > passes_max) passes_max = p;
+        passes += p;
         sg++; i = j;
     }
-    Seg32 *dseg = (Seg32 *)stage(0, (size_t)segs * sizeof(Seg32));
-    void *xd = stage(1, xbytes); float *yd = (float *)stage(2, ybytes); uint32_t *dmap = (uint32_t *)stage(3, (size_t)M * 4);
-    if (!dseg || !xd || !yd || !dmap) { free(hseg); return OMEGA_GPU_FP8GEMM_CHIP_FAIL; }
     cudaStream_t s = g.stream;
-    bool ok = cuda_ok(cudaMemcpyAsync(dseg, hseg, (size_t)segs * sizeof(Seg32), cudaMemcpyHostToDevice, s), "copy segments") &&
-              cuda_ok(cudaMemcpyAsync(dmap, trow, (size_t)M * 4, cudaMemcpyHostToDevice, s), "copy row table") &&
-              cuda_ok(cudaMemcpyAsync(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, cudaMemcpyHostToDevice, s), "copy x") &&
-              cuda_ok(cudaStreamSynchronize(s), "stage");
-    free(hseg);
-    if (!ok) return OMEGA_GPU_FP8GEMM_CHIP_FAIL;
-    launch_fill_f32(yd, (size_t)M * n, POISON_F32, s);
+    char *dt = (char *)stage(0, tables.size()); void *xd = stage(1, xbytes);
+    HostResult r;
+    if (!dt || !xd || !to_device(dt, tables.data(), tables.size(), s) || !to_device(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, s) ||
+        !r.open((size_t)M * n, s)) return OMEGA_GPU_FP8GEMM_CHIP_FAIL;
     GemvArgs a = {};
-    a.seg = dseg; a.x = xd; a.x_bf16 = x16 ? 1 : 0; a.x_rows = x_rows; a.xmap = dmap; a.ymap = nullptr;
-    a.y = yd; a.n = n; a.k = k; a.groups_or_segs = segs; a.rows = M; a.out_mul = 1.0f; a.mutant = g.gemm_mutant;
-    uint32_t gx = 0, mt = 0;
-    cudaEventRecord(g.ev0, s);
-    ok = cuda_ok(launch_gemm_rows(a, &gx, &mt, s), "fp8gemm launch");
-    cudaEventRecord(g.ev1, s);
-    float *yh = (float *)malloc(ybytes);
-    if (!yh) return OMEGA_GPU_FP8GEMM_BAD_ARGS;
-    ok = ok && cuda_ok(cudaMemcpyAsync(yh, yd, ybytes, cudaMemcpyDeviceToHost, s), "copy y") && cuda_ok(cudaStreamSynchronize(s), "fp8gemm");
-    int rc = ok ? OMEGA_GPU_FP8GEMM_OK : OMEGA_GPU_FP8GEMM_CHIP_FAIL;
-    if (ok) {
-        size_t unchanged = 0;
-        for (size_t i = 0; i < (size_t)M * n; i++) if (yh[i] == POISON_F32) unchanged++;
-        if (unchanged) { set_error("output poison survived"); rc = OMEGA_GPU_FP8GEMM_CHIP_FAIL; }
-        else memcpy(y, yh, ybytes);
-    }
-    free(yh);
+    a.seg = (const Seg32 *)dt; a.x = xd; a.x_bf16 = x16 ? 1 : 0; a.x_rows = x_rows; a.xmap = (const uint32_t *)(dt + sbytes); a.ymap = nullptr;
+    a.y = r.dev; a.n = n; a.k = k; a.groups_or_segs = segs; a.rows = M; a.out_mul = 1.0f; a.mutant = g.gemm_mutant;
+    uint32_t gx = 0;
+    if (info) cudaEventRecord(g.ev0, s);
+    const bool ok = cuda_ok(launch_gemm_rows(a, &gx, nullptr, s), "fp8gemm launch");
+    if (info) cudaEventRecord(g.ev1, s);
+    const int rc = ok ? r.take(y, info != nullptr, "fp8gemm") : OMEGA_GPU_FP8GEMM_CHIP_FAIL;
     if (info) {
         const uint32_t lb = k % 512u == 0 ? 16u : k % 256u == 0 ? 8u : 4u;
-        info->rows = M; info->segments = segs; info->n = n; info->k = k; info->mt = mt; info->warps_per_cta = 8; info->lane_bytes = lb;
-        info->grid_x = gx; info->grid_y = segs; info->passes_max = passes_max;
-        info->weight_bytes = (uint64_t)segs * n * k; info->streamed_bytes = streamed; info->kernel_cache_hit = true;
+        info->rows = M; info->segments = segs; info->n = n; info->k = k; info->mt = mt; info->warps_per_cta = ROWS_WARPS; info->lane_bytes = lb;
+        info->grid_x = gx; info->grid_y = segs; info->passes_max = (uint32_t)passes_max;
+        info->weight_bytes = (uint64_t)segs * n * k; info->streamed_bytes = passes * n * k; info->kernel_cache_hit = true;
         info->general = lb == 4u;
         if (ok) { float ms = 0; if (cudaEventElapsedTime(&ms, g.ev0, g.ev1) == cudaSuccess) info->elapsed_ns = (uint64_t)(ms * 1e6); info->completion_marker = 1; }
         info->call_ns = now_ns() - t0;

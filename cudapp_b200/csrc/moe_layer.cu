@@ -36,8 +36,9 @@ static Workspace *workspace_create(uint32_t max_tokens, uint32_t topk, uint32_t 
     const size_t max_tiles = R / 8 + experts + 8;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += align_up(bytes); return o; };
-    const size_t o_ids = take(R * 4), o_wts = take(R * 4), o_cnt = take((size_t)experts * 4), o_st = take((size_t)experts * 4),
-                 o_xm = take(Rp * 4), o_ym = take(Rp * 4), o_hdr = take(64), o_sgu = take((size_t)experts * 32), o_sdn = take((size_t)experts * 32),
+    // header, ids and weights first and together: the host entry reads them back as one block
+    const size_t o_hdr = take(64), o_ids = take(R * 4), o_wts = take(R * 4), o_cnt = take((size_t)experts * 4), o_st = take((size_t)experts * 4),
+                 o_xm = take(Rp * 4), o_ym = take(Rp * 4), o_sgu = take((size_t)experts * 32), o_sdn = take((size_t)experts * 32),
                  o_tiles = take(max_tiles * 16), o_gu = take(Rp * 2 * inter * 4), o_act = take(Rp * inter * 4), o_dn = take(Rp * hidden * 4),
                  o_qx = take(Rp * 4 * hidden), o_qa = take(Rp * 4 * inter), o_sx = take(Rp * (hidden / 128) * 4), o_sa = take(Rp * (inter / 128) * 4),
                  o_lg = take((size_t)max_tokens * experts * 2), o_x = take((size_t)max_tokens * hidden * 2), o_o16 = take((size_t)max_tokens * hidden * 2),
@@ -340,15 +341,21 @@ int omega_gpu_moe_layer_bf16(OmegaGpuMoeLayer *L, uint32_t tokens, const uint16_
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
     Workspace *w = L->ws; cudaStream_t s = st().stream;
     const size_t lb = (size_t)tokens * (L->experts - L->shared) * 2, xb = (size_t)tokens * L->hidden * 2, rb = (size_t)tokens * L->cfg.topk * 4;
-    bool ok = cuda_ok(cudaMemcpyAsync(w->logits, logits, lb, cudaMemcpyHostToDevice, s), "copy logits") &&
-              cuda_ok(cudaMemcpyAsync(w->x, x, xb, cudaMemcpyHostToDevice, s), "copy x") &&
-              layer_forward(L, tokens, w->logits, w->x, w->out32, w->out16, s);
-    if (ok && out_bf16) ok = cuda_ok(cudaMemcpyAsync(out_bf16, w->out16, xb, cudaMemcpyDeviceToHost, s), "copy out");
-    if (ok && out_f32) ok = cuda_ok(cudaMemcpyAsync(out_f32, w->out32, xb * 2, cudaMemcpyDeviceToHost, s), "copy out");
-    if (ok && ids) ok = cuda_ok(cudaMemcpyAsync(ids, w->ids, rb, cudaMemcpyDeviceToHost, s), "copy ids");
-    if (ok && wts) ok = cuda_ok(cudaMemcpyAsync(wts, w->wts, rb, cudaMemcpyDeviceToHost, s), "copy weights");
+    bool ok = to_device(w->logits, logits, lb, s) && to_device(w->x, x, xb, s) && layer_forward(L, tokens, w->logits, w->x, w->out32, w->out16, s);
+    if (ok && out_bf16) ok = to_host(out_bf16, w->out16, xb, s);
+    if (ok && out_f32) ok = to_host(out_f32, w->out32, xb * 2, s);
+    // header, ids and weights: one copy when they fit the result area
+    char *area = ok ? (char *)result_area() : nullptr;
+    const size_t block = (size_t)((char *)w->wts - (char *)w->header) + rb;
+    const bool together = block <= RESULT_BYTES;
+    ok = ok && area && cuda_ok(cudaMemcpyAsync(area, w->header, together ? block : 32, cudaMemcpyDeviceToHost, s), "copy status");
+    if (ok && !together && ids) ok = to_host(ids, w->ids, rb, s);
+    if (ok && !together && wts) ok = to_host(wts, w->wts, rb, s);
+    ok = ok && cuda_ok(cudaStreamSynchronize(s), "moe layer");
     uint32_t hdr[8] = {0};
-    ok = ok && cuda_ok(cudaMemcpyAsync(hdr, w->header, 32, cudaMemcpyDeviceToHost, s), "copy status") && cuda_ok(cudaStreamSynchronize(s), "moe layer");
+    if (ok) memcpy(hdr, area, 32);
+    if (ok && together && ids) memcpy(ids, area + ((char *)w->ids - (char *)w->header), rb);
+    if (ok && together && wts) memcpy(wts, area + ((char *)w->wts - (char *)w->header), rb);
     if (ok && hdr[3]) { set_error("moe layer: routing plan refused (status %u)", hdr[3]); return OMEGA_GPU_FP8_BAD_ARGS; }
     if (ok && hdr[4]) { set_error("moe layer: a bounded wait inside the tensor-core kernel ran out (code %u)", hdr[4]); st().latched = true; return OMEGA_GPU_FP8_CHIP_FAIL; }
     return ok ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;

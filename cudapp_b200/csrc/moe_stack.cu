@@ -433,11 +433,10 @@ int omega_gpu_moe_stack_bf16(OmegaGpuMoeStack *S, uint32_t tokens, const uint16_
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
     cudaStream_t s = st().stream;
     const size_t xb = (size_t)tokens * S->hidden * 2, lb = S->layers.size() * (size_t)tokens * (S->experts - S->shared) * 2;
-    bool ok = (S->router_mode || cuda_ok(cudaMemcpyAsync(S->logits, logits, lb, cudaMemcpyHostToDevice, s), "copy logits")) &&
-              cuda_ok(cudaMemcpyAsync(S->x, x, xb, cudaMemcpyHostToDevice, s), "copy x") &&
+    bool ok = (S->router_mode || to_device(S->logits, logits, lb, s)) && to_device(S->x, x, xb, s) &&
               stack_run(S, tokens, S->logits, S->x, nullptr, S->out16, s);
-    if (ok && out_bf16) ok = cuda_ok(cudaMemcpyAsync(out_bf16, S->out16, xb, cudaMemcpyDeviceToHost, s), "copy out");
-    if (ok && out_f32) ok = cuda_ok(cudaMemcpyAsync(out_f32, S->h, xb * 2, cudaMemcpyDeviceToHost, s), "copy out");
+    if (ok && out_bf16) ok = to_host(out_bf16, S->out16, xb, s);
+    if (ok && out_f32) ok = to_host(out_f32, S->h, xb * 2, s);
     std::vector<uint32_t> hdr;
     if (ok && S->fused) { hdr.resize(S->layers.size() * 8); ok = cuda_ok(cudaMemcpyAsync(hdr.data(), S->pb.header, hdr.size() * 4, cudaMemcpyDeviceToHost, s), "copy status"); }
     ok = ok && cuda_ok(cudaStreamSynchronize(s), "moe stack");

@@ -94,14 +94,14 @@ int omega_gpu_moe_w4_layer_bf16(OmegaGpuMoeW4Layer *L, uint32_t tokens, const ui
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
     cudaStream_t s = st().stream;
     const size_t lb = (size_t)tokens * L->experts * 2, xb = (size_t)tokens * L->hidden * 2, rb = (size_t)tokens * L->topk * 4;
-    bool ok = cuda_ok(cudaMemcpyAsync(L->logits, logits_bf16, lb, cudaMemcpyHostToDevice, s), "copy logits") && cuda_ok(cudaMemcpyAsync(L->x, x_bf16, xb, cudaMemcpyHostToDevice, s), "copy x");
+    bool ok = to_device(L->logits, logits_bf16, lb, s) && to_device(L->x, x_bf16, xb, s);
     if (!ok) return OMEGA_GPU_FP8_CHIP_FAIL;
     const int rc = omega_gpu_moe_w4_layer_async(L, tokens, (uint64_t)(uintptr_t)L->logits, (uint64_t)(uintptr_t)L->x, (uint64_t)(uintptr_t)L->out32, (uint64_t)(uintptr_t)L->out16, s);
     if (rc != OMEGA_GPU_FP8_OK) return rc;
-    if (out_bf16) ok = ok && cuda_ok(cudaMemcpyAsync(out_bf16, L->out16, xb, cudaMemcpyDeviceToHost, s), "copy out");
-    if (out_f32) ok = ok && cuda_ok(cudaMemcpyAsync(out_f32, L->out32, xb * 2, cudaMemcpyDeviceToHost, s), "copy out");
-    if (ids) ok = ok && cuda_ok(cudaMemcpyAsync(ids, L->ids, rb, cudaMemcpyDeviceToHost, s), "copy ids");
-    if (wts) ok = ok && cuda_ok(cudaMemcpyAsync(wts, L->wts, rb, cudaMemcpyDeviceToHost, s), "copy weights");
+    if (out_bf16) ok = ok && to_host(out_bf16, L->out16, xb, s);
+    if (out_f32) ok = ok && to_host(out_f32, L->out32, xb * 2, s);
+    if (ids) ok = ok && to_host(ids, L->ids, rb, s);
+    if (wts) ok = ok && to_host(wts, L->wts, rb, s);
     uint32_t hdr[8] = {0};
     ok = ok && cuda_ok(cudaMemcpyAsync(hdr, L->header, 32, cudaMemcpyDeviceToHost, s), "copy status") && cuda_ok(cudaStreamSynchronize(s), "w4 layer");
     if (ok && hdr[3]) { set_error("w4 layer: routing plan refused (status %u)", hdr[3]); return OMEGA_GPU_FP8_BAD_ARGS; }

@@ -61,6 +61,59 @@ void *stage(int i, size_t bytes) {
     return g.stage[i];
 }
 
+constexpr size_t RING_CHUNK = 256 * 1024, INLINE_COPY = 64 * 1024; constexpr int RING = 4;
+static bool pinned_open() {
+    State &g = st();
+    if (g.pinned) return true;
+    for (auto &e : g.ring_ev) if (!e && !cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate")) return false;
+    void *p = nullptr;
+    if (!cuda_ok(cudaHostAlloc(&p, RING * RING_CHUNK + RESULT_BYTES + 64, cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc(staging)")) return false;
+    g.pinned = (char *)p;
+    return true;
+}
+void *result_area() { return pinned_open() ? st().pinned + RING * RING_CHUNK : nullptr; }
+bool host_pinned(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeHost;
+}
+bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    if (bytes <= INLINE_COPY || host_pinned(src)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "copy to the device");
+    if (!pinned_open()) return false;
+    State &g = st();
+    int i = 0;
+    for (size_t at = 0; at < bytes; at += RING_CHUNK, i = (i + 1) % RING) {
+        const size_t n = bytes - at < RING_CHUNK ? bytes - at : RING_CHUNK;
+        char *slot = g.pinned + i * RING_CHUNK;
+        if (!cuda_ok(cudaEventSynchronize(g.ring_ev[i]), "staging chunk")) return false;   // its last DMA, of this call or an earlier one
+        memcpy(slot, (const char *)src + at, n);
+        if (!cuda_ok(cudaMemcpyAsync((char *)dst + at, slot, n, cudaMemcpyHostToDevice, s), "copy to the device") || !cuda_ok(cudaEventRecord(g.ring_ev[i], s), "event")) return false;
+    }
+    return true;
+}
+bool to_host(void *dst, const void *src, size_t bytes, cudaStream_t s, const volatile uint32_t *stop) {
+    if (host_pinned(dst)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "copy to the host");
+    if (!pinned_open()) return false;
+    State &g = st();
+    const size_t chunks = (bytes + RING_CHUNK - 1) / RING_CHUNK;
+    auto len = [&](size_t c) { const size_t left = bytes - c * RING_CHUNK; return left < RING_CHUNK ? left : RING_CHUNK; };
+    auto queue = [&](size_t c) {
+        const int i = (int)(c % RING);
+        return cuda_ok(cudaEventSynchronize(g.ring_ev[i]), "staging chunk") &&
+               cuda_ok(cudaMemcpyAsync(g.pinned + i * RING_CHUNK, (const char *)src + c * RING_CHUNK, len(c), cudaMemcpyDeviceToHost, s), "copy to the host") &&
+               cuda_ok(cudaEventRecord(g.ring_ev[i], s), "event");
+    };
+    for (size_t c = 0; c < chunks && c < (size_t)RING; c++) if (!queue(c)) return false;
+    for (size_t c = 0; c < chunks; c++) {
+        const int i = (int)(c % RING);
+        if (!cuda_ok(cudaEventSynchronize(g.ring_ev[i]), "copy to the host")) return false;
+        if (stop && *stop) return true;
+        memcpy((char *)dst + c * RING_CHUNK, g.pinned + i * RING_CHUNK, len(c));
+        if (c + RING < chunks && !queue(c + RING)) return false;
+    }
+    return true;
+}
+
 __global__ void fill_f32_kernel(float *p, size_t n, float v) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
 }
@@ -129,6 +182,15 @@ __global__ void scan_codes_kernel(const uint8_t *w, size_t wbytes, const uint16_
 using namespace b200;
 
 extern "C" {
+
+int omega_gpu_host_alloc(uint64_t bytes, void **out) {
+    if (out) *out = nullptr;
+    if (!bytes || !out) return OMEGA_GPU_FP8_BAD_ARGS;
+    Lock l;
+    if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
+    return cuda_ok(cudaHostAlloc(out, bytes, cudaHostAllocPortable), "cudaHostAlloc") ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;
+}
+void omega_gpu_host_free(void *p) { if (p) { Lock l; (void)cudaFreeHost(p); } }
 
 const char *omega_gpu_fp8_rc_name(int rc) {
     switch (rc) {

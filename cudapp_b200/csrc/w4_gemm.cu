@@ -457,9 +457,9 @@ int omega_gpu_w4_gemm_bf16(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t
     uint16_t *dx = (uint16_t *)stage(0, xb), *d16 = (uint16_t *)stage(1, yb * 2); float *d32 = (float *)stage(2, yb * 4);
     if (!dx || !d16 || !d32) return OMEGA_GPU_FP8_CHIP_FAIL;
     cudaStream_t s = st().stream;
-    bool ok = cuda_ok(cudaMemcpyAsync(dx, x, xb, cudaMemcpyHostToDevice, s), "copy x") && cuda_ok(w4_launch(t, m, dx, d16, d32, s), "w4 launch");
-    if (ok && y16) ok = cuda_ok(cudaMemcpyAsync(y16, d16, yb * 2, cudaMemcpyDeviceToHost, s), "copy y");
-    if (ok && y32) ok = cuda_ok(cudaMemcpyAsync(y32, d32, yb * 4, cudaMemcpyDeviceToHost, s), "copy y");
+    bool ok = to_device(dx, x, xb, s) && cuda_ok(w4_launch(t, m, dx, d16, d32, s), "w4 launch");
+    if (ok && y16) ok = to_host(y16, d16, yb * 2, s);
+    if (ok && y32) ok = to_host(y32, d32, yb * 4, s);
     ok = ok && cuda_ok(cudaStreamSynchronize(s), "w4 gemm");
     return ok ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;
 }

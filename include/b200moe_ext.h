@@ -21,6 +21,11 @@ int omega_gpu_fp8_tensor_upload_dev(uint32_t experts, uint32_t n, uint32_t k, ui
                                     OmegaGpuFp8Tensor **out);
 int omega_gpu_fp8_quantize_bf16_dev(uint32_t n, uint32_t k, uint64_t w_bf16_va, uint64_t w8_va, uint64_t scale_inv_bf16_va);
 
+/* ---- page-locked host memory for the buffers of the host entries: results and inputs in it travel by DMA as they are, pageable ones pass through
+ * a staging ring. Any host memory is accepted everywhere; this only saves the extra copy. */
+int omega_gpu_host_alloc(uint64_t bytes, void **out);
+void omega_gpu_host_free(void *p);
+
 /* ---- router top-k on given logits: k rounds of "largest remaining, lowest index on ties", ids in selection order,
  * weights = softmax over the selected logits (norm_topk) or over all experts (src/omega_blackwell_codegen_router.c:298-401,
  * oracle tests/gpu_router_test.c:62-79). logits bf16 [tokens][experts], experts <= 1024, topk <= 32. */
