@@ -2,8 +2,8 @@
 // columns) times bf16 activations, f32 accumulation, bf16 output. The reference has no integer-W4 arithmetic
 // (docs/models/QUANT.md:62 of the reference: "integer W4 refuses"), so this follows the benchmark definition only:
 // y[m][r] = sum over groups g of scale[r][g] * sum_{c in g} x[m][c] * q[r][c].
-// Two kernels. The tensor-core kernel takes the shapes it is written for (n a multiple of 128; k 1024, 2048 or 4096); the
-// CUDA-core kernel takes every other shape: a warp owns RW output rows; lane l owns K groups l, l+32, ... (16 contiguous bytes
+// Three kernels. The tensor-core kernels take the shapes they are written for (n a multiple of 128; k 768, 1024, 2048 or 4096), one up to 16 rows (and a routing plan's tiles), the
+// other more; the CUDA-core kernel takes every other shape: a warp owns RW output rows; lane l owns K groups l, l+32, ... (16 contiguous bytes
 // each, 512 contiguous bytes per warp load); the activation panel sits in shared memory as bf16.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -125,11 +125,14 @@ __device__ __forceinline__ void e2m1x8_bf16(uint32_t v, uint32_t *b) {
     }
 }
 
+// unsigned E4M3: (8 + m) * 2^(e - 10) for e > 0 (binary32 exponent field e + 120), m * 2^-9 for e = 0
+__device__ __forceinline__ float ue4m3_f32(uint32_t c) { return (c >> 3) ? __uint_as_float((((c >> 3) + 120u) << 23) | ((c & 7u) << 20)) : (float)(c & 7u) * 0.001953125f; }
+
 // FMT 2 (NVFP4: E2M1 + one unsigned E4M3 scale per 16 columns): a 32-column group holds two scale groups, so its two MMAs must be columns 0..15 and
 // 16..31. Thread t of a quad then feeds columns 4t .. 4t+3 to the first MMA and 16+4t .. 16+4t+3 to the second: the two 16-bit halves it needs sit in
 // the words of quad threads t/2 and 2 + t/2 (one shuffle each); each MMA goes into its own fresh accumulator and is scaled by its own scale.
 template <int GQ, int FMT>   // 32-column groups per K quarter: k = 128 * GQ; FMT 0: int4 + fp16 scales, 1: E2M1 + E8M0 scales (MXFP4), 2: E2M1 + UE4M3 per 16 (NVFP4)
-__global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t m0, uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint16_t *__restrict__ sc,
+__global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint16_t *__restrict__ sc,
                                                         const uint16_t *__restrict__ x, uint16_t *__restrict__ y16, float *__restrict__ y32, float *part, uint32_t *counters,
                                                         const uint4 *__restrict__ tiles, const uint32_t *__restrict__ header, const uint32_t *__restrict__ xmap, const uint32_t *__restrict__ ymap) {
     constexpr uint32_t KQ = GQ * 32u, XS = KQ * 2u + 64u;   // columns per quarter; bytes between panel rows (the 64 keep a quarter-warp's 16-byte reads on separate banks)
@@ -138,14 +141,14 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
     const uint32_t nb = blockIdx.x, kq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, t = lane & 3u;
     // grouped form (tiles != null): blockIdx.z is a row tile {expert, first sorted row, rows <= 16} of a routing plan; the tensor holds the experts' matrices
     // one after the other (n rows each); activation row i of the tile is x[xmap[row0 + i]] (or row0 + i), its result goes to row ymap[row0 + i] (or row0 + i)
-    uint32_t mt = 0, row0 = m0;
+    uint32_t mt = 0, row0 = 0;
     if (tiles) {
         if (blockIdx.z >= header[2]) return;
         const uint4 tl = tiles[blockIdx.z];
         w += (size_t)tl.x * n * (k / 2u); sc = reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(sc) + (size_t)tl.x * n * (k / 32u) * (FMT == 1 ? 1u : 2u));
         row0 = tl.y; mt = min(16u, tl.z);
         part += (size_t)blockIdx.z * 4u * 16u * n; counters += (size_t)blockIdx.z * (n / 128u);
-    } else mt = min(16u, m - m0);
+    } else mt = m;
     // this thread's weight words: output row n0 + r, word t of every group of the quarter; all requested before anything else
     const uint32_t n0 = nb * 128u + warp * 8u;
     const uint32_t *wrow = reinterpret_cast<const uint32_t *>(w + (size_t)(n0 + r) * (k / 2u) + (size_t)kq * (KQ / 2u));
@@ -171,7 +174,7 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
             reinterpret_cast<uint16_t *>(&sv1[0])[i] = __ldg(reinterpret_cast<const uint16_t *>(s1b) + i);
         }
     }
-    // the quarter of the activation panel: rows m0 .. m0 + 15 (zero past m), columns kq * KQ ..
+    // the quarter of the activation panel: 16 rows (zero past the last), columns kq * KQ ..
     for (uint32_t i = threadIdx.x; i < 16u * (KQ / 8u); i += 512u) {
         const uint32_t row = i / (KQ / 8u), c8 = i - row * (KQ / 8u);
         uint4 v = make_uint4(0, 0, 0, 0);
@@ -195,9 +198,7 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
             mma_bf16_16816(p2, xc.x, xd.x, xc.y, xd.y, bq[2], bq[3]);
             const uint32_t *u0 = reinterpret_cast<const uint32_t *>(&sv0[g >> 3]), *u1 = reinterpret_cast<const uint32_t *>(&sv1[g >> 3]);
             const uint32_t h0 = (u0[(g & 7) >> 1] >> (16 * (g & 1))) & 0xffffu, h1 = (u1[(g & 7) >> 1] >> (16 * (g & 1))) & 0xffffu;
-            // unsigned E4M3: (8 + m) * 2^(e - 10) for e > 0 (binary32 exponent field e + 120), m * 2^-9 for e = 0
-            auto ue4m3 = [](uint32_t c) -> float { return (c >> 3) ? __uint_as_float((((c >> 3) + 120u) << 23) | ((c & 7u) << 20)) : (float)(c & 7u) * 0.001953125f; };
-            const float a0 = ue4m3(h0 & 0xffu), a1 = ue4m3(h0 >> 8), c0 = ue4m3(h1 & 0xffu), c1 = ue4m3(h1 >> 8);
+            const float a0 = ue4m3_f32(h0 & 0xffu), a1 = ue4m3_f32(h0 >> 8), c0 = ue4m3_f32(h1 & 0xffu), c1 = ue4m3_f32(h1 >> 8);
             acc[0] = fmaf(p[0], a0, acc[0]); acc[1] = fmaf(p[1], c0, acc[1]); acc[2] = fmaf(p[2], a0, acc[2]); acc[3] = fmaf(p[3], c0, acc[3]);
             acc[0] = fmaf(p2[0], a1, acc[0]); acc[1] = fmaf(p2[1], c1, acc[1]); acc[2] = fmaf(p2[2], a1, acc[2]); acc[3] = fmaf(p2[3], c1, acc[3]);
             continue;
@@ -239,6 +240,181 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
         if (y16) { const uint32_t b = __float_as_uint(v); y16[at] = (uint16_t)(((b & 0x7fffffffu) > 0x7f800000u) ? ((b >> 16) | 0x40u) : ((b + 0x7fffu + ((b >> 16) & 1u)) >> 16)); }
     }
     if (threadIdx.x == 0) counters[nb] = 0;   // ready for the next launch (launches on one tensor are stream-ordered)
+}
+
+// ---------------------------------------------------------------- tensor-core kernel for more than 16 activation rows
+// Taken 16 rows a launch by the kernel above, m rows read and decode every weight m / 16 times, in launches that follow one another. Here a decoded
+// weight fragment meets MT row tiles of 16 before it is dropped, and one launch covers all rows: the work is bound by the mma.sync rate and by how
+// often x is read again from L2 (once per 16 * NT columns). The sums are those of the kernel above, bit for bit: a group's two MMAs start from zero,
+// its scale joins in f32, groups of a K quarter in order, then the quarters in order; so a row's result does not depend on how many rows came with it.
+// CTA: 16 * MT rows x 16 * NT columns, eight warps = four K quarters x two halves of the columns; a warp holds MT x NT m16n8 accumulators over its
+// quarter. A step is two scale groups of every quarter: rows of x (64 columns), weights (two 16-byte groups a row) and scales (4 bytes a row) come by
+// cp.async into one of two stages while the other is used. Two CTAs per SM (128 registers). The 16-byte chunks of a row of x are permuted by
+// bits 0 and 1 of the row, so that a quad's fragments of neighbouring rows fall on different banks.
+// Measured with a cold L2 against launches of 16 rows (int4 / MXFP4 / NVFP4): 300 x 4096 x 2048 169 / 171 / 205 -> 49 / 51 / 61 us, 17 x 4096 x 2048
+// 21.5 / 21.5 / 25.6 -> 14.3 us, 512 x 8192 x 4096 698 / 756 / 916 -> 215 / 227 / 270 us.
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, uint32_t bytes) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)); }
+__device__ __forceinline__ void cp4(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src)); }
+__device__ __forceinline__ uint32_t w4_chunk(uint32_t row, uint32_t c) { return c ^ (((row & 1u) << 2) | (row & 2u)); }
+__device__ __forceinline__ void mma_bf16_zero(float *d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ void mma_bf16_add(float *d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__host__ __device__ constexpr uint32_t w4_rows_stage(int MT, int NT) { return MT * 8192u + NT * 2048u + NT * 256u; }   // bytes: x, weights, scales of one step
+constexpr uint32_t w4_rows_smem(int MT, int NT) {
+    const uint32_t red = 4u * MT * 16u * (16u * NT + 8u) * 4u, st = 2u * w4_rows_stage(MT, NT);     // the quarters' sums reuse the stages
+    return red > st ? red : st;
+}
+
+template <int FMT, int MT, int NT>
+__global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint8_t *__restrict__ sc,
+                                                             const uint16_t *__restrict__ x, uint16_t *__restrict__ y16, float *__restrict__ y32) {
+    constexpr uint32_t ROWS = MT * 16u, COLS = NT * 16u, WOFF = MT * 8192u, SOFF = WOFF + NT * 2048u, STAGE = w4_rows_stage(MT, NT), RS = COLS + 8u;
+    constexpr uint32_t SB = FMT == 1 ? 1u : 2u;   // scale bytes per 32 columns
+    extern __shared__ __align__(16) uint8_t sm[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, t = lane & 3u, kq = warp >> 1, half = warp & 1u;
+    const uint32_t ct = n / COLS, m0 = blockIdx.x / ct * ROWS, n0 = blockIdx.x % ct * COLS, GQ = k / 128u, steps = GQ / 2u, srow = k / 32u * SB;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+    auto load = [&](uint32_t step, uint32_t st) {
+        const uint32_t b = base + st * STAGE;
+#pragma unroll 1
+        for (uint32_t row = threadIdx.x >> 3; row < ROWS; row += 32u) {   // not unrolled: the addresses would take the registers of the sums
+            const uint32_t c = threadIdx.x & 7u, dst = b + row * 128u + w4_chunk(row, c) * 16u;
+            const bool in = m0 + row < m;
+            const uint16_t *src = x + (size_t)(in ? m0 + row : m0) * k + step * 64u + c * 8u;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) cp16(dst + q * ROWS * 128u, src + q * (k / 4u), in ? 16u : 0u);
+        }
+#pragma unroll
+        for (uint32_t i = threadIdx.x; i < 4u * 2u * COLS; i += 256u) {   // [quarter][group][column]
+            const uint32_t q = i / (2u * COLS), col = (i >> 1) % COLS, g = i & 1u;
+            cp16(b + WOFF + ((q * 2u + g) * COLS + col) * 16u, w + (size_t)(n0 + col) * (k / 2u) + q * (k / 8u) + (step * 2u + g) * 16u, 16u);
+        }
+        if (threadIdx.x < 4u * COLS) {   // one byte per group: the aligned word that holds this step's two
+            const uint32_t q = threadIdx.x / COLS, col = threadIdx.x % COLS;
+            cp4(b + SOFF + threadIdx.x * 4u, sc + (size_t)(n0 + col) * srow + ((q * GQ + step * 2u) * SB & ~3u));
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    float acc[MT][NT][4];
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) { acc[i][j][0] = 0.0f; acc[i][j][1] = 0.0f; acc[i][j][2] = 0.0f; acc[i][j][3] = 0.0f; }
+    load(0, 0);
+    for (uint32_t step = 0; step < steps; step++) {
+        if (step + 1u < steps) { load(step + 1u, (step + 1u) & 1u); asm volatile("cp.async.wait_group 1;"); }
+        else asm volatile("cp.async.wait_group 0;");
+        __syncthreads();
+        const uint8_t *b = sm + (step & 1u) * STAGE, *xs = b + kq * ROWS * 128u;
+        const uint32_t *ws = reinterpret_cast<const uint32_t *>(b + WOFF) + (kq * 2u * COLS + half * 8u * NT) * 4u;
+        const uint32_t *ss = reinterpret_cast<const uint32_t *>(b + SOFF) + kq * COLS + half * 8u * NT;
+#pragma unroll
+        for (uint32_t g = 0; g < 2; g++) {
+            uint32_t bq[NT][4]; float s0[NT][SB], s1[NT][SB];   // scales of columns 2t and 2t + 1 (FMT 2: of either half of the group)
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const uint32_t *wr = ws + (g * COLS + j * 8u + r) * 4u;
+                if (FMT == 2) {
+                    const uint32_t wa = wr[t >> 1], wb = wr[2u + (t >> 1)];
+                    e2m1x8_bf16((t & 1u) ? ((wa >> 16) | (wb & 0xffff0000u)) : ((wa & 0xffffu) | (wb << 16)), bq[j]);
+                } else if (FMT == 1) e2m1x8_bf16(wr[t], bq[j]);
+                else {
+                    const uint32_t v = wr[t];
+                    bq[j][0] = nib2_bf16(v, 0); bq[j][1] = nib2_bf16(v, 1); bq[j][2] = nib2_bf16(v, 2); bq[j][3] = nib2_bf16(v, 3);
+                }
+                const uint2 sv = *reinterpret_cast<const uint2 *>(ss + j * 8u + 2u * t);
+                if (FMT == 1) {
+                    const uint32_t sh = ((kq * GQ + step * 2u) & 2u) * 8u + 8u * g, e0 = (sv.x >> sh) & 0xffu, e1 = (sv.y >> sh) & 0xffu;
+                    s0[j][0] = __uint_as_float(e0 ? e0 << 23 : 0x00400000u); s1[j][0] = __uint_as_float(e1 ? e1 << 23 : 0x00400000u);
+                } else {
+                    const uint32_t h0 = (sv.x >> (16 * g)) & 0xffffu, h1 = (sv.y >> (16 * g)) & 0xffffu;
+                    if (FMT == 0) { s0[j][0] = __half2float(__ushort_as_half((unsigned short)h0)); s1[j][0] = __half2float(__ushort_as_half((unsigned short)h1)); }
+                    else { s0[j][0] = ue4m3_f32(h0 & 0xffu); s0[j][SB - 1] = ue4m3_f32(h0 >> 8); s1[j][0] = ue4m3_f32(h1 & 0xffu); s1[j][SB - 1] = ue4m3_f32(h1 >> 8); }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < MT; i++) {
+                const uint32_t row = i * 16u + r;   // row + 8 has the same permutation
+                if (FMT == 2) {
+                    const uint8_t *pa = xs + row * 128u + w4_chunk(row, g * 4u + (t >> 1)) * 16u + (t & 1u) * 8u, *pc = xs + row * 128u + w4_chunk(row, g * 4u + 2u + (t >> 1)) * 16u + (t & 1u) * 8u;
+                    const uint2 xa = *reinterpret_cast<const uint2 *>(pa), xb = *reinterpret_cast<const uint2 *>(pa + 1024), xc = *reinterpret_cast<const uint2 *>(pc), xd = *reinterpret_cast<const uint2 *>(pc + 1024);
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        float p[4], p2[4], *a = acc[i][j];
+                        mma_bf16_zero(p, xa.x, xb.x, xa.y, xb.y, bq[j][0], bq[j][1]);
+                        mma_bf16_zero(p2, xc.x, xd.x, xc.y, xd.y, bq[j][2], bq[j][3]);
+                        a[0] = fmaf(p[0], s0[j][0], a[0]); a[1] = fmaf(p[1], s1[j][0], a[1]); a[2] = fmaf(p[2], s0[j][0], a[2]); a[3] = fmaf(p[3], s1[j][0], a[3]);
+                        a[0] = fmaf(p2[0], s0[j][SB - 1], a[0]); a[1] = fmaf(p2[1], s1[j][SB - 1], a[1]); a[2] = fmaf(p2[2], s0[j][SB - 1], a[2]); a[3] = fmaf(p2[3], s1[j][SB - 1], a[3]);
+                    }
+                } else {
+                    const uint8_t *pa = xs + row * 128u + w4_chunk(row, g * 4u + t) * 16u;
+                    const uint4 xa = *reinterpret_cast<const uint4 *>(pa), xb = *reinterpret_cast<const uint4 *>(pa + 1024);
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        float p[4], *a = acc[i][j];
+                        mma_bf16_zero(p, xa.x, xb.x, xa.y, xb.y, bq[j][0], bq[j][1]);
+                        mma_bf16_add(p, xa.z, xb.z, xa.w, xb.w, bq[j][2], bq[j][3]);
+                        a[0] = fmaf(p[0], s0[j][0], a[0]); a[1] = fmaf(p[1], s1[j][0], a[1]); a[2] = fmaf(p[2], s0[j][0], a[2]); a[3] = fmaf(p[3], s1[j][0], a[3]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    float *red = reinterpret_cast<float *>(sm);   // [quarter][row][RS]
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            float *o = red + (kq * ROWS + i * 16u + r) * RS + half * 8u * NT + j * 8u + 2u * t;
+            *reinterpret_cast<float2 *>(o) = make_float2(acc[i][j][0], acc[i][j][1]);
+            *reinterpret_cast<float2 *>(o + 8u * RS) = make_float2(acc[i][j][2], acc[i][j][3]);
+        }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < ROWS * COLS; i += 256u) {
+        const uint32_t row = i / COLS, col = i % COLS;
+        if (m0 + row >= m) break;
+        float v = red[row * RS + col];
+#pragma unroll
+        for (uint32_t q = 1; q < 4; q++) v = __fadd_rn(v, red[(q * ROWS + row) * RS + col]);
+        const size_t at = (size_t)(m0 + row) * n + n0 + col;
+        if (y32) y32[at] = v;
+        if (y16) { const uint32_t u = __float_as_uint(v); y16[at] = (uint16_t)(((u & 0x7fffffffu) > 0x7f800000u) ? ((u >> 16) | 0x40u) : ((u + 0x7fffu + ((u >> 16) & 1u)) >> 16)); }
+    }
+}
+
+template <int FMT, int MT, int NT>
+static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
+    // set on every call: it belongs to the device's context and costs well under a launch
+    const cudaError_t e = cudaFuncSetAttribute(w4_mma_rows_kernel<FMT, MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4_rows_smem(MT, NT));
+    if (e != cudaSuccess) return e;
+    w4_mma_rows_kernel<FMT, MT, NT><<<dim3(t->n / (16u * NT) * ((m + 16u * MT - 1u) / (16u * MT))), 256, w4_rows_smem(MT, NT), s>>>(m, t->n, t->k, t->w, reinterpret_cast<const uint8_t *>(t->s), dx, d16, d32);
+    return cudaGetLastError();
+}
+template <int FMT>
+static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
+    // Few CTAs want small tiles, many want tall ones (a decoded weight is used more often); in between the number of waves decides. The cost of a tile is its
+    // MT x NT products, its decoding (NT) and a fixed part. Measured (int4): 17 x 4096 x 2048 14.3 us at 2 x 2 and 26.6 at 4 x 4; 512 x 8192 x 4096 215 us at
+    // 4 x 4 and 268 at 2 x 2; 300 x 4096 x 2048 49 us at 5 x 4 (one wave, although some of its sums spill) and 55 at 4 x 4 (two waves).
+    const uint32_t slots = 2u * (uint32_t)(st().sm_count ? st().sm_count : 148), tiles = (m + 15u) / 16u;
+    uint32_t best = 0, cost = ~0u;
+    for (uint32_t c = 0; c < 5; c++) {   // MT 2, 3, 4, 5 with NT = 4, then MT = 2 with NT = 2
+        const uint32_t mt = c < 4u ? c + 2u : 2u, nt = c < 4u ? 4u : 2u;
+        const uint32_t waves = (t->n / (16u * nt) * ((tiles + mt - 1u) / mt) + slots - 1u) / slots, v = waves * (mt * nt + nt + 4u);
+        if (v < cost) { cost = v; best = c; }
+    }
+    switch (best) {
+    case 0: return w4_rows_start<FMT, 2, 4>(t, m, dx, d16, d32, s);
+    case 1: return w4_rows_start<FMT, 3, 4>(t, m, dx, d16, d32, s);
+    case 2: return w4_rows_start<FMT, 4, 4>(t, m, dx, d16, d32, s);
+    case 3: return w4_rows_start<FMT, 5, 4>(t, m, dx, d16, d32, s);
+    default: return w4_rows_start<FMT, 2, 2>(t, m, dx, d16, d32, s);
+    }
 }
 
 // NVFP4 block quantiser (the reference's native/models/nvfp4.om: nvfp4nib = nvfp4scale + nvfp4enc per element). One thread per 16-element block of a
@@ -284,7 +460,7 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
 cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     const dim3 grid(t->gn / 128u, 4, t->gtiles);
-#define W4_GROUPED(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(0u, 0u, t->gn, t->k, t->w, t->s, dx, d16, d32, t->gpart, t->gcounters, \
+#define W4_GROUPED(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(0u, t->gn, t->k, t->w, t->s, dx, d16, d32, t->gpart, t->gcounters, \
         (const uint4 *)tiles, header, xmap, ymap)
     if (t->fmt == 2) { if (t->k == 4096u) W4_GROUPED(32, 2); else if (t->k == 2048u) W4_GROUPED(16, 2); else if (t->k == 1024u) W4_GROUPED(8, 2); else W4_GROUPED(6, 2); }
     else if (t->fmt) { if (t->k == 4096u) W4_GROUPED(32, 1); else if (t->k == 2048u) W4_GROUPED(16, 1); else if (t->k == 1024u) W4_GROUPED(8, 1); else W4_GROUPED(6, 1); }
@@ -400,15 +576,14 @@ void omega_gpu_w4_free(OmegaGpuW4Tensor *t) {
     free(t);
 }
 static cudaError_t w4_launch(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
-    if (t->part && (t->fmt || !getenv("B200MOE_W4_FMA"))) {   // tensor-core kernel: one launch per 16 activation rows (they share the tensor's scratch, in stream order)
+    if (t->part && (t->fmt || !getenv("B200MOE_W4_FMA"))) {   // tensor-core kernels
+        if (m > 16u) return t->fmt == 2 ? w4_rows<2>(t, m, dx, d16, d32, s) : t->fmt ? w4_rows<1>(t, m, dx, d16, d32, s) : w4_rows<0>(t, m, dx, d16, d32, s);
         const dim3 grid(t->n / 128u, 4);
-        for (uint32_t m0 = 0; m0 < m; m0 += 16u) {
-#define W4_LAUNCH(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(m0, m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters, nullptr, nullptr, nullptr, nullptr)
-            if (t->fmt == 2) { if (t->k == 4096u) W4_LAUNCH(32, 2); else if (t->k == 2048u) W4_LAUNCH(16, 2); else if (t->k == 1024u) W4_LAUNCH(8, 2); else W4_LAUNCH(6, 2); }
-            else if (t->fmt) { if (t->k == 4096u) W4_LAUNCH(32, 1); else if (t->k == 2048u) W4_LAUNCH(16, 1); else if (t->k == 1024u) W4_LAUNCH(8, 1); else W4_LAUNCH(6, 1); }
-            else { if (t->k == 4096u) W4_LAUNCH(32, 0); else if (t->k == 2048u) W4_LAUNCH(16, 0); else if (t->k == 1024u) W4_LAUNCH(8, 0); else W4_LAUNCH(6, 0); }
+#define W4_LAUNCH(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters, nullptr, nullptr, nullptr, nullptr)
+        if (t->fmt == 2) { if (t->k == 4096u) W4_LAUNCH(32, 2); else if (t->k == 2048u) W4_LAUNCH(16, 2); else if (t->k == 1024u) W4_LAUNCH(8, 2); else W4_LAUNCH(6, 2); }
+        else if (t->fmt) { if (t->k == 4096u) W4_LAUNCH(32, 1); else if (t->k == 2048u) W4_LAUNCH(16, 1); else if (t->k == 1024u) W4_LAUNCH(8, 1); else W4_LAUNCH(6, 1); }
+        else { if (t->k == 4096u) W4_LAUNCH(32, 0); else if (t->k == 2048u) W4_LAUNCH(16, 0); else if (t->k == 1024u) W4_LAUNCH(8, 0); else W4_LAUNCH(6, 0); }
 #undef W4_LAUNCH
-        }
         return cudaGetLastError();
     }
     const size_t smem = (size_t)W4_MT * t->k * 2;
