@@ -87,6 +87,26 @@ inline volatile uint32_t *result_flag(void *area) { return reinterpret_cast<vola
 
 struct Lock { Lock() { st().mu.lock(); } ~Lock() { st().mu.unlock(); } };
 
+// ---- programmatic dependent launch: the kernel may be set up while the one before it in the stream still runs, so that a chain of short kernels does not
+// pay a launch gap each. Every kernel launched this way begins with griddep_chain: it waits until the grids before it have completed and their
+// writes are visible, and only then lets the next kernel start. So at any time only neighbours in the chain overlap, and a kernel that looks at
+// older results ahead of its own wait (the expert kernel reads the plan) finds them complete. Results of earlier kernels are read with plain loads
+// (no __restrict__ on const inputs, no __ldg): a load marked as invariant may be moved ahead of the wait.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {}; cudaLaunchAttribute at[1];
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void griddep_chain() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // ---- launchers implemented across the .cu files (all stream-ordered, device pointers)
 // y poison / generic fill
 void launch_fill_f32(float *p, size_t n, float v, cudaStream_t s);
@@ -121,10 +141,11 @@ cudaError_t launch_swiglu(uint32_t rows, uint32_t inter, const float *gu, float 
 cudaError_t launch_combine(uint32_t tokens, uint32_t slots, uint32_t hidden, const float *w, const float *d, float *out_f32, uint16_t *out_bf16, cudaStream_t s);
 // quantise rows of x (f32 or bf16; gathered through xmap when given) into e4m3 pieces: q [rows][pieces][k], s [rows][k/128]
 cudaError_t launch_act_quant(uint32_t rows, uint32_t k, uint32_t pieces, const void *x, int x_bf16, const uint32_t *xmap,
-                             const uint32_t *rows_dev, uint8_t *q, float *sc, cudaStream_t s, size_t x_stride_bytes = 0, uint32_t q_rows = 0);
+                             const uint32_t *rows_dev, uint8_t *q, float *sc, cudaStream_t s, size_t x_stride_bytes = 0, uint32_t q_rows = 0,
+                             uint32_t *clear = nullptr, uint32_t clear_words = 0);   // clear: words set to zero on the way (the expert kernel's work list)
 // sorted row r <- codes (all pieces, piece-major with src_rows / dst_rows rows per piece) and scales of source row xmap[r]
 cudaError_t launch_gather_rows(uint32_t rows, uint32_t k, uint32_t pieces, uint32_t src_rows, uint32_t dst_rows, const uint32_t *xmap, const uint32_t *rows_dev,
-                               const uint8_t *q_src, const float *s_src, uint8_t *q_dst, float *s_dst, cudaStream_t s);
+                               const uint8_t *q_src, const float *s_src, uint8_t *q_dst, float *s_dst, cudaStream_t s, uint32_t *clear = nullptr, uint32_t clear_words = 0);
 // tcgen05 grouped GEMM (fp8_mma_sm100.cu)
 struct MmaLaunch {
     const float *wscale, *ascale;      // weight scales [E][n/128][k/128]; activation scales [rows][k/128]

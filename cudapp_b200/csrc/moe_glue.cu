@@ -10,7 +10,8 @@ namespace b200 {
 // (src/omega_blackwell_codegen_dec.c:291-324).
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdiv_rn(g, 1.0f + expf(-g)) * u; }
 
-__global__ void __launch_bounds__(256) swiglu_kernel(uint32_t rows, uint32_t inter, const float *__restrict__ gu, float *__restrict__ act, uint16_t *__restrict__ act16) {
+__global__ void __launch_bounds__(256) swiglu_kernel(uint32_t rows, uint32_t inter, const float *gu, float *__restrict__ act, uint16_t *__restrict__ act16) {
+    griddep_chain();
     const size_t total = (size_t)rows * inter;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / inter, c = i - r * inter;
@@ -23,14 +24,14 @@ cudaError_t launch_swiglu(uint32_t rows, uint32_t inter, const float *gu, float 
     const size_t total = (size_t)rows * inter;
     if (!total) return cudaSuccess;
     size_t blocks = (total + 255) / 256; if (blocks > 148 * 8) blocks = 148 * 8;
-    swiglu_kernel<<<(unsigned)blocks, 256, 0, s>>>(rows, inter, gu, act, act_bf16);
-    return cudaGetLastError();
+    return launch_chained(swiglu_kernel, dim3((unsigned)blocks), dim3(256), 0, s, rows, inter, gu, act, act_bf16);
 }
 
 // out[t][c] = w0*d0 ; then m = m + w_s*d_s for s = 1.. in slot order, multiply and add kept separate
 // (src/omega_blackwell_codegen_dec.c:226-255: FMUL then FADD, never FFMA).
-__global__ void __launch_bounds__(256) combine_kernel(uint32_t tokens, uint32_t slots, uint32_t hidden, const float *__restrict__ w,
-                                                      const float *__restrict__ d, float *__restrict__ out, uint16_t *__restrict__ out_bf16) {
+__global__ void __launch_bounds__(256) combine_kernel(uint32_t tokens, uint32_t slots, uint32_t hidden, const float *w,
+                                                      const float *d, float *__restrict__ out, uint16_t *__restrict__ out_bf16) {
+    griddep_chain();
     const uint32_t t = blockIdx.x;
     for (uint32_t c = threadIdx.x * 4; c < hidden; c += blockDim.x * 4) {
         const float4 m = combine_slots<false>(slots, w, d, (size_t)t * slots, hidden, c);
@@ -45,16 +46,16 @@ __global__ void __launch_bounds__(256) combine_kernel(uint32_t tokens, uint32_t 
 }
 cudaError_t launch_combine(uint32_t tokens, uint32_t slots, uint32_t hidden, const float *w, const float *d, float *out_f32, uint16_t *out_bf16, cudaStream_t s) {
     if (!tokens) return cudaSuccess;
-    combine_kernel<<<tokens, 256, 0, s>>>(tokens, slots, hidden, w, d, out_f32, out_bf16);
-    return cudaGetLastError();
+    return launch_chained(combine_kernel, dim3(tokens), dim3(256), 0, s, tokens, slots, hidden, w, d, out_f32, out_bf16);
 }
 
 // Activation quantiser: quant_pieces_warp (mma_common.cuh) applied to rows of x. One warp per (row, 128-column group); lane = 4 columns.
-__global__ void __launch_bounds__(256) act_quant_kernel(uint32_t rows, uint32_t k, uint32_t pieces, size_t piece_stride, const void *__restrict__ x, int x_bf16, size_t x_stride,
-                                                        const uint32_t *__restrict__ xmap, const uint32_t *__restrict__ rows_dev,
-                                                        uint8_t *__restrict__ q, float *__restrict__ sc) {
-    // a kernel launched as a programmatic dependent of this one (the expert kernel: it fetches weights and waits for this grid before it reads a row) may start now
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__global__ void __launch_bounds__(256) act_quant_kernel(uint32_t rows, uint32_t k, uint32_t pieces, size_t piece_stride, const void *x, int x_bf16, size_t x_stride,
+                                                        const uint32_t *xmap, const uint32_t *rows_dev,
+                                                        uint8_t *__restrict__ q, float *__restrict__ sc, uint32_t *__restrict__ clear, uint32_t clear_words) {
+    // after the wait the expert kernel may start: it reads the plan, which is complete by then, fetches weights and waits for this grid before it reads a row
+    griddep_chain();
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear_words; i += gridDim.x * blockDim.x) clear[i] = 0;
     const uint32_t lane = threadIdx.x & 31u, kb = k / 128u;
     const uint32_t nrows = rows_dev ? min(rows, *rows_dev) : rows;
     const uint32_t tasks = nrows * kb, stride = gridDim.x * (blockDim.x >> 5);   // rows <= 2^24 and kb <= 32 on every caller's path
@@ -69,10 +70,10 @@ __global__ void __launch_bounds__(256) act_quant_kernel(uint32_t rows, uint32_t 
             rr[u] = r; bb[u] = b;
             const uint32_t src = xmap ? xmap[r] : r;
             if (x_bf16) {
-                const uint2 w = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint8_t *>(x) + (size_t)src * x_stride + (b * 128u + lane * 4u) * 2u));
+                const uint2 w = *reinterpret_cast<const uint2 *>(reinterpret_cast<const uint8_t *>(x) + (size_t)src * x_stride + (b * 128u + lane * 4u) * 2u);
                 v[u][0] = __uint_as_float(w.x << 16); v[u][1] = __uint_as_float(w.x & 0xffff0000u); v[u][2] = __uint_as_float(w.y << 16); v[u][3] = __uint_as_float(w.y & 0xffff0000u);
             } else {
-                const float4 w = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const uint8_t *>(x) + (size_t)src * x_stride + (b * 128u + lane * 4u) * 4u));
+                const float4 w = *reinterpret_cast<const float4 *>(reinterpret_cast<const uint8_t *>(x) + (size_t)src * x_stride + (b * 128u + lane * 4u) * 4u);
                 v[u][0] = w.x; v[u][1] = w.y; v[u][2] = w.z; v[u][3] = w.w;
             }
         }
@@ -89,23 +90,24 @@ __global__ void __launch_bounds__(256) act_quant_kernel(uint32_t rows, uint32_t 
 }
 // q: piece p of row r at q[p * q_rows * k + r * k] (piece-major; q_rows = row capacity, 0 = rows)
 cudaError_t launch_act_quant(uint32_t rows, uint32_t k, uint32_t pieces, const void *x, int x_bf16, const uint32_t *xmap, const uint32_t *rows_dev,
-                             uint8_t *q, float *sc, cudaStream_t s, size_t x_stride_bytes, uint32_t q_rows) {
+                             uint8_t *q, float *sc, cudaStream_t s, size_t x_stride_bytes, uint32_t q_rows, uint32_t *clear, uint32_t clear_words) {
     if (!q_rows) q_rows = rows;
     if (!x_stride_bytes) x_stride_bytes = (size_t)k * (x_bf16 ? 2 : 4);
     const size_t tasks = (size_t)rows * (k / 128u);
     if (!tasks) return cudaSuccess;
     if (tasks >= ((size_t)1 << 32)) return cudaErrorInvalidValue;
     size_t blocks = (tasks + 7) / 8; if (blocks > 148 * 8) blocks = 148 * 8;
-    act_quant_kernel<<<(unsigned)blocks, 256, 0, s>>>(rows, k, pieces, (size_t)q_rows * k, x, x_bf16, x_stride_bytes, xmap, rows_dev, q, sc);
-    return cudaGetLastError();
+    return launch_chained(act_quant_kernel, dim3((unsigned)blocks), dim3(256), 0, s, rows, k, pieces, (size_t)q_rows * k, x, x_bf16, x_stride_bytes, xmap, rows_dev, q, sc, clear, clear_words);
 }
 
 // Sorted-row copies of rows that were quantised once per source row: sorted row r takes the codes (every piece) and the scales of
 // source row xmap[r]. One warp per (sorted row, piece); k is a multiple of 128, so a row is k / 16 16-byte words.
 __global__ void __launch_bounds__(256) gather_rows_kernel(uint32_t rows, uint32_t k, uint32_t pieces, size_t src_piece_stride, size_t dst_piece_stride,
-                                                          const uint32_t *__restrict__ xmap, const uint32_t *__restrict__ rows_dev,
-                                                          const uint8_t *__restrict__ q_src, const float *__restrict__ s_src, uint8_t *__restrict__ q_dst, float *__restrict__ s_dst) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // as in act_quant_kernel
+                                                          const uint32_t *xmap, const uint32_t *rows_dev,
+                                                          const uint8_t *q_src, const float *s_src, uint8_t *__restrict__ q_dst, float *__restrict__ s_dst,
+                                                          uint32_t *__restrict__ clear, uint32_t clear_words) {
+    griddep_chain();   // as in act_quant_kernel
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear_words; i += gridDim.x * blockDim.x) clear[i] = 0;
     const uint32_t lane = threadIdx.x & 31u, kb = k / 128u, words = k / 16u;
     const uint32_t nrows = rows_dev ? min(rows, *rows_dev) : rows;
     const uint32_t tasks = nrows * pieces, stride = gridDim.x * (blockDim.x >> 5);
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(uint32_t rows, uint32_
         for (uint32_t w0 = 0; w0 < words; w0 += 128u) {   // four independent 16-byte loads per lane before the first store
             uint4 v[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) { const uint32_t w = w0 + lane + 32u * i; v[i] = w < words ? __ldg(from + w) : make_uint4(0, 0, 0, 0); }
+            for (int i = 0; i < 4; i++) { const uint32_t w = w0 + lane + 32u * i; v[i] = w < words ? from[w] : make_uint4(0, 0, 0, 0); }
 #pragma unroll
             for (int i = 0; i < 4; i++) { const uint32_t w = w0 + lane + 32u * i; if (w < words) to[w] = v[i]; }
         }
@@ -124,13 +126,13 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(uint32_t rows, uint32_
     }
 }
 cudaError_t launch_gather_rows(uint32_t rows, uint32_t k, uint32_t pieces, uint32_t src_rows, uint32_t dst_rows, const uint32_t *xmap, const uint32_t *rows_dev,
-                               const uint8_t *q_src, const float *s_src, uint8_t *q_dst, float *s_dst, cudaStream_t s) {
+                               const uint8_t *q_src, const float *s_src, uint8_t *q_dst, float *s_dst, cudaStream_t s, uint32_t *clear, uint32_t clear_words) {
     const size_t tasks = (size_t)rows * pieces;
     if (!tasks) return cudaSuccess;
     if (tasks >= ((size_t)1 << 32)) return cudaErrorInvalidValue;
     size_t blocks = (tasks + 7) / 8; if (blocks > 148 * 8) blocks = 148 * 8;
-    gather_rows_kernel<<<(unsigned)blocks, 256, 0, s>>>(rows, k, pieces, (size_t)src_rows * k, (size_t)dst_rows * k, xmap, rows_dev, q_src, s_src, q_dst, s_dst);
-    return cudaGetLastError();
+    return launch_chained(gather_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, s, rows, k, pieces, (size_t)src_rows * k, (size_t)dst_rows * k, xmap, rows_dev, q_src, s_src, q_dst, s_dst,
+                          clear, clear_words);
 }
 
 }  // namespace b200

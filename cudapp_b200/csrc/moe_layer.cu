@@ -115,22 +115,21 @@ bool layer_forward(OmegaGpuMoeLayer *L, uint32_t tokens, const uint16_t *logits,
         // activations as e4m3 pieces in sorted-row order, then the two tensor-core grouped GEMMs
         const uint32_t Px = L->cfg.x_pieces, Pa = L->cfg.act_pieces, Rp = w->max_tokens * w->topk + 8;
         uint32_t extra_q = 0;
-        if (!cuda_ok(cudaMemsetAsync(w->sched, 0, (size_t)w->sched_words * 4, s), "clear work list")) return false;   // the one-launch expert kernel's tickets and tile counters
         if (K >= 4u && tokens >= 512u) {
             // many picks per token: quantise every token row once, then copy codes and scales into sorted-row order (the same bytes as
             // quantising each sorted row, a fraction of the arithmetic)
             if (!cuda_ok(launch_act_quant(tokens, H, Px, x, 1, nullptr, nullptr, w->qt, w->stt, s, 0, w->max_tokens), "x quant launch") ||
-                !cuda_ok(launch_gather_rows(R, H, Px, w->max_tokens, Rp, w->xmap, w->header, w->qt, w->stt, w->qx, w->sx, s), "x gather launch")) return false;
+                !cuda_ok(launch_gather_rows(R, H, Px, w->max_tokens, Rp, w->xmap, w->header, w->qt, w->stt, w->qx, w->sx, s, w->sched, w->sched_words), "x gather launch")) return false;
             extra_q = 1;
-        } else if (!cuda_ok(launch_act_quant(R, H, Px, x, 1, w->xmap, w->header, w->qx, w->sx, s, 0, Rp), "x quant launch")) return false;
+        } else if (!cuda_ok(launch_act_quant(R, H, Px, x, 1, w->xmap, w->header, w->qx, w->sx, s, 0, Rp, w->sched, w->sched_words), "x quant launch")) return false;
         MARK("x_quant");
-        // decode-shaped calls: the whole expert FFN in one launch (gate|up units, then down units from a work list cleared just before)
+        // decode-shaped calls: the whole expert FFN in one launch (gate|up units, then down units from the work list that the kernel before it cleared)
         static const bool two_launches = getenv("B200MOE_TWO_LAUNCH") != nullptr;
         if (!wide && !two_launches && ffn_shape_ok(H, I) && ((Px == 2 && Pa == 3) || (Px == 1 && Pa == 1) || (Px == 2 && Pa == 2))) {
             FfnLaunch f = {};
             f.gu_scale = L->gu->s; f.dn_scale = L->dn->s; f.x_scale = w->sx; f.qa = w->qa; f.sa = w->sa; f.tiles = w->tiles; f.header = w->header; f.ymap = w->ymap;
             f.out = w->dn; f.hidden = H; f.inter = I; f.q_rows = Rp; f.sched = w->sched; f.err = w->header + 4;
-            // programmatic dependent of the quantiser before it (the work list was cleared ahead of that kernel): set-up and first weight tiles overlap it
+            // programmatic dependent of the quantiser before it (which also cleared the work list): set-up and first weight tiles overlap it
             if (!cuda_ok(launch_ffn(L->tm_gu, L->tm_qx, L->tm_dn, L->tm_qa, Px, Pa, f, s, true), "expert ffn launch")) return false;
             MARK("expert_ffn_mma");
             if (!cuda_ok(launch_combine(tokens, K, H, w->wts, w->dn, out32, out16, s), "combine launch")) return false; MARK("combine");

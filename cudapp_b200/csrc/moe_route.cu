@@ -17,7 +17,8 @@ namespace b200 {
 // slots = entries per token in ids / wts: topk, or topk + 1 when a shared expert follows the routed picks (its id = experts, weight 1:
 // the reference's ninth group, src/omega_gpu_q36_graph.h:7-21; a caller with a shared-expert gate supplies the weight through the router)
 __global__ void __launch_bounds__(256) topk_kernel(uint32_t tokens, uint32_t experts, uint32_t topk, int norm, uint32_t slots,
-                                                   const uint16_t *__restrict__ logits, uint32_t *__restrict__ ids, float *__restrict__ wts) {
+                                                   const uint16_t *logits, uint32_t *__restrict__ ids, float *__restrict__ wts) {
+    griddep_chain();
     extern __shared__ float sm[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, t = blockIdx.x * (blockDim.x >> 5) + warp;
     if (t >= tokens) return;
@@ -30,8 +31,7 @@ __global__ void __launch_bounds__(256) topk_kernel(uint32_t tokens, uint32_t exp
 
 cudaError_t launch_topk(uint32_t tokens, uint32_t experts, uint32_t topk, int norm, const uint16_t *logits, uint32_t *ids, float *wts, cudaStream_t s, uint32_t slots) {
     const uint32_t warps = experts <= 512 ? 8u : 4u;
-    topk_kernel<<<(tokens + warps - 1) / warps, warps * 32, (size_t)warps * experts * 4, s>>>(tokens, experts, topk, norm, slots ? slots : topk, logits, ids, wts);
-    return cudaGetLastError();
+    return launch_chained(topk_kernel, dim3((tokens + warps - 1) / warps), dim3(warps * 32), (size_t)warps * experts * 4, s, tokens, experts, topk, norm, slots ? slots : topk, logits, ids, wts);
 }
 
 // ------------------------------------------------------------------ plan: one CTA of 1024 threads
@@ -110,7 +110,7 @@ __device__ __forceinline__ bool plan_tables(uint32_t experts, uint32_t tile_rows
 // dynamic shared: counts[E] | starts[E] | run[E] | scan buf[96] | wcnt u16 [32][E]
 // pos (optional): inverse of the Y map, pos[token * slots + slot] = sorted row of that pick
 __device__ __forceinline__ void plan_body(uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows,
-                                          const uint32_t *__restrict__ ids, const OmegaGpuMoePlanOut &o, uint32_t *__restrict__ pos) {
+                                          const uint32_t *ids, const OmegaGpuMoePlanOut &o, uint32_t *__restrict__ pos) {
     extern __shared__ uint32_t smem[];
     uint32_t *counts = smem, *starts = smem + experts, *run = smem + 2 * experts, *sbuf = smem + 3 * experts;
     uint16_t *wcnt = reinterpret_cast<uint16_t *>(sbuf + 96);
@@ -159,12 +159,14 @@ __device__ __forceinline__ void plan_body(uint32_t tokens, uint32_t slots, uint3
 }
 
 __global__ void __launch_bounds__(1024) plan_kernel(uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows,
-                                                    const uint32_t *__restrict__ ids, const OmegaGpuMoePlanOut o) {
+                                                    const uint32_t *ids, const OmegaGpuMoePlanOut o) {
+    griddep_chain();
     plan_body(tokens, slots, experts, ystride, tile_rows, ids, o, nullptr);
 }
 // one CTA per layer: layer l's picks at ids + l * tokens * slots, its outputs at the PlanBatch strides
 __global__ void __launch_bounds__(1024) plan_batch_kernel(uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows,
-                                                          const uint32_t *__restrict__ ids, const PlanBatch b) {
+                                                          const uint32_t *ids, const PlanBatch b) {
+    griddep_chain();
     const uint32_t l = blockIdx.x;
     OmegaGpuMoePlanOut o = {};
     o.counts_va = (uint64_t)(uintptr_t)(b.counts + (size_t)l * experts); o.starts_va = (uint64_t)(uintptr_t)(b.starts + (size_t)l * experts);
@@ -179,15 +181,15 @@ cudaError_t launch_plan_batch(uint32_t layers, uint32_t tokens, uint32_t slots, 
         cudaError_t e = cudaFuncSetAttribute(plan_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    plan_batch_kernel<<<layers, 1024, smem, s>>>(tokens, slots, experts, ystride, tile_rows, ids, b);
-    return cudaGetLastError();
+    return launch_chained(plan_batch_kernel, dim3(layers), dim3(1024), smem, s, tokens, slots, experts, ystride, tile_rows, ids, b);
 }
 
 // ------------------------------------------------------------------ plan of many picks: three launches, one CTA per 1024 picks in the first and the last
 // The same stable order as plan_kernel (sorted row = rows of lower experts + earlier picks of the same expert), split so that the
 // per-chunk work runs on as many SMs as there are chunks: (1) per-chunk histograms, (2) one CTA turns them into per-chunk
 // offsets and builds the tables, (3) every chunk scatters its picks. scratch: u32 [chunks][experts] + 1 flag word.
-__global__ void __launch_bounds__(1024) plan_hist_kernel(uint32_t R, uint32_t experts, const uint32_t *__restrict__ ids, uint32_t *__restrict__ scratch, uint32_t chunks) {
+__global__ void __launch_bounds__(1024) plan_hist_kernel(uint32_t R, uint32_t experts, const uint32_t *ids, uint32_t *__restrict__ scratch, uint32_t chunks) {
+    griddep_chain();
     extern __shared__ uint32_t smem[];
     const uint32_t tid = threadIdx.x;
     for (uint32_t e = tid; e < experts; e += 1024) smem[e] = 0;
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(1024) plan_hist_kernel(uint32_t R, uint32_t ex
 }
 // dynamic shared: counts[E] | starts[E] | scan buf[96]
 __global__ void __launch_bounds__(1024) plan_scan_kernel(uint32_t experts, uint32_t tile_rows, uint32_t *__restrict__ scratch, uint32_t chunks, const OmegaGpuMoePlanOut o) {
+    griddep_chain();
     extern __shared__ uint32_t smem[];
     uint32_t *counts = smem, *starts = smem + experts, *sbuf = smem + 2 * experts;
     const uint32_t tid = threadIdx.x;
@@ -217,8 +220,9 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(uint32_t experts, uint3
     (void)plan_tables(experts, tile_rows, counts, starts, sbuf, o, bad);
 }
 // dynamic shared: wcnt u16 [32][E]
-__global__ void __launch_bounds__(1024) plan_scatter_kernel(uint32_t R, uint32_t slots, uint32_t experts, uint32_t ystride, const uint32_t *__restrict__ ids,
-                                                            const uint32_t *__restrict__ scratch, const OmegaGpuMoePlanOut o, uint32_t *__restrict__ pos) {
+__global__ void __launch_bounds__(1024) plan_scatter_kernel(uint32_t R, uint32_t slots, uint32_t experts, uint32_t ystride, const uint32_t *ids,
+                                                            const uint32_t *scratch, const OmegaGpuMoePlanOut o, uint32_t *__restrict__ pos) {
+    griddep_chain();
     extern __shared__ uint32_t smem[];
     uint16_t *wcnt = reinterpret_cast<uint16_t *>(smem);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -257,10 +261,10 @@ cudaError_t launch_plan(uint32_t tokens, uint32_t slots, uint32_t experts, uint3
                         const OmegaGpuMoePlanOut &o, cudaStream_t s, uint32_t *scratch, size_t scratch_words) {
     const uint32_t R = tokens * slots, chunks = (R + 1023u) / 1024u;
     if (plan_split(R, experts, scratch, scratch_words, o)) {
-        plan_hist_kernel<<<chunks, 1024, (size_t)experts * 4, s>>>(R, experts, ids, scratch, chunks);
-        plan_scan_kernel<<<1, 1024, (size_t)experts * 8 + 96 * 4, s>>>(experts, tile_rows, scratch, chunks, o);
-        plan_scatter_kernel<<<chunks, 1024, (size_t)32 * experts * 2, s>>>(R, slots, experts, ystride, ids, scratch, o, nullptr);
-        return cudaGetLastError();
+        cudaError_t e = launch_chained(plan_hist_kernel, dim3(chunks), dim3(1024), (size_t)experts * 4, s, R, experts, ids, scratch, chunks);
+        if (e == cudaSuccess) e = launch_chained(plan_scan_kernel, dim3(1), dim3(1024), (size_t)experts * 8 + 96 * 4, s, experts, tile_rows, scratch, chunks, o);
+        if (e == cudaSuccess) e = launch_chained(plan_scatter_kernel, dim3(chunks), dim3(1024), (size_t)32 * experts * 2, s, R, slots, experts, ystride, ids, scratch, o, nullptr);
+        return e;
     }
 
     const size_t smem = (size_t)experts * 12 + 96 * 4 + (size_t)32 * experts * 2;
@@ -268,8 +272,7 @@ cudaError_t launch_plan(uint32_t tokens, uint32_t slots, uint32_t experts, uint3
         cudaError_t e = cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    plan_kernel<<<1, 1024, smem, s>>>(tokens, slots, experts, ystride, tile_rows, ids, o);
-    return cudaGetLastError();
+    return launch_chained(plan_kernel, dim3(1), dim3(1024), smem, s, tokens, slots, experts, ystride, tile_rows, ids, o);
 }
 
 }  // namespace b200

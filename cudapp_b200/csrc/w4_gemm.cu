@@ -133,8 +133,8 @@ __device__ __forceinline__ float ue4m3_f32(uint32_t c) { return (c >> 3) ? __uin
 // the words of quad threads t/2 and 2 + t/2 (one shuffle each); each MMA goes into its own fresh accumulator and is scaled by its own scale.
 template <int GQ, int FMT>   // 32-column groups per K quarter: k = 128 * GQ; FMT 0: int4 + fp16 scales, 1: E2M1 + E8M0 scales (MXFP4), 2: E2M1 + UE4M3 per 16 (NVFP4)
 __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint16_t *__restrict__ sc,
-                                                        const uint16_t *__restrict__ x, uint16_t *__restrict__ y16, float *__restrict__ y32, float *part, uint32_t *counters,
-                                                        const uint4 *__restrict__ tiles, const uint32_t *__restrict__ header, const uint32_t *__restrict__ xmap, const uint32_t *__restrict__ ymap) {
+                                                        const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32, float *part, uint32_t *counters,
+                                                        const uint4 *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap) {
     constexpr uint32_t KQ = GQ * 32u, XS = KQ * 2u + 64u;   // columns per quarter; bytes between panel rows (the 64 keep a quarter-warp's 16-byte reads on separate banks)
     extern __shared__ __align__(16) uint8_t xq[];
     __shared__ uint32_t s_last;
@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
     // one after the other (n rows each); activation row i of the tile is x[xmap[row0 + i]] (or row0 + i), its result goes to row ymap[row0 + i] (or row0 + i)
     uint32_t mt = 0, row0 = 0;
     if (tiles) {
+        griddep_chain();
         if (blockIdx.z >= header[2]) return;
         const uint4 tl = tiles[blockIdx.z];
         w += (size_t)tl.x * n * (k / 2u); sc = reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(sc) + (size_t)tl.x * n * (k / 32u) * (FMT == 1 ? 1u : 2u));
@@ -174,11 +175,12 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
             reinterpret_cast<uint16_t *>(&sv1[0])[i] = __ldg(reinterpret_cast<const uint16_t *>(s1b) + i);
         }
     }
+    if (!tiles) griddep_chain();   // the weights are the tensor's own: only what follows depends on earlier work
     // the quarter of the activation panel: 16 rows (zero past the last), columns kq * KQ ..
     for (uint32_t i = threadIdx.x; i < 16u * (KQ / 8u); i += 512u) {
         const uint32_t row = i / (KQ / 8u), c8 = i - row * (KQ / 8u);
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < mt) v = __ldg(reinterpret_cast<const uint4 *>(x + (size_t)(xmap ? xmap[row0 + row] : row0 + row) * k + (size_t)kq * KQ) + c8);
+        if (row < mt) v = reinterpret_cast<const uint4 *>(x + (size_t)(xmap ? xmap[row0 + row] : row0 + row) * k + (size_t)kq * KQ)[c8];
         *reinterpret_cast<uint4 *>(xq + row * XS + c8 * 16u) = v;
     }
     __syncthreads();
@@ -272,7 +274,8 @@ constexpr uint32_t w4_rows_smem(int MT, int NT) {
 
 template <int FMT, int MT, int NT>
 __global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint8_t *__restrict__ sc,
-                                                             const uint16_t *__restrict__ x, uint16_t *__restrict__ y16, float *__restrict__ y32) {
+                                                             const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32) {
+    griddep_chain();
     constexpr uint32_t ROWS = MT * 16u, COLS = NT * 16u, WOFF = MT * 8192u, SOFF = WOFF + NT * 2048u, STAGE = w4_rows_stage(MT, NT), RS = COLS + 8u;
     constexpr uint32_t SB = FMT == 1 ? 1u : 2u;   // scale bytes per 32 columns
     extern __shared__ __align__(16) uint8_t sm[];
@@ -393,8 +396,8 @@ static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, const ui
     // set on every call: it belongs to the device's context and costs well under a launch
     const cudaError_t e = cudaFuncSetAttribute(w4_mma_rows_kernel<FMT, MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4_rows_smem(MT, NT));
     if (e != cudaSuccess) return e;
-    w4_mma_rows_kernel<FMT, MT, NT><<<dim3(t->n / (16u * NT) * ((m + 16u * MT - 1u) / (16u * MT))), 256, w4_rows_smem(MT, NT), s>>>(m, t->n, t->k, t->w, reinterpret_cast<const uint8_t *>(t->s), dx, d16, d32);
-    return cudaGetLastError();
+    return launch_chained(w4_mma_rows_kernel<FMT, MT, NT>, dim3(t->n / (16u * NT) * ((m + 16u * MT - 1u) / (16u * MT))), dim3(256), w4_rows_smem(MT, NT), s,
+                          m, t->n, t->k, t->w, reinterpret_cast<const uint8_t *>(t->s), dx, d16, d32);
 }
 template <int FMT>
 static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
@@ -460,13 +463,12 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
 cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     const dim3 grid(t->gn / 128u, 4, t->gtiles);
-#define W4_GROUPED(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(0u, t->gn, t->k, t->w, t->s, dx, d16, d32, t->gpart, t->gcounters, \
-        (const uint4 *)tiles, header, xmap, ymap)
+#define W4_GROUPED(GQV, FMTV) return launch_chained(w4_mma_kernel<GQV, FMTV>, grid, dim3(512), 16 * (GQV * 64 + 64), s, 0u, t->gn, t->k, t->w, t->s, dx, d16, d32, t->gpart, \
+        t->gcounters, (const uint4 *)tiles, header, xmap, ymap)
     if (t->fmt == 2) { if (t->k == 4096u) W4_GROUPED(32, 2); else if (t->k == 2048u) W4_GROUPED(16, 2); else if (t->k == 1024u) W4_GROUPED(8, 2); else W4_GROUPED(6, 2); }
     else if (t->fmt) { if (t->k == 4096u) W4_GROUPED(32, 1); else if (t->k == 2048u) W4_GROUPED(16, 1); else if (t->k == 1024u) W4_GROUPED(8, 1); else W4_GROUPED(6, 1); }
     else { if (t->k == 4096u) W4_GROUPED(32, 0); else if (t->k == 2048u) W4_GROUPED(16, 0); else if (t->k == 1024u) W4_GROUPED(8, 0); else W4_GROUPED(6, 0); }
 #undef W4_GROUPED
-    return cudaGetLastError();
 }
 
 }  // namespace b200
@@ -579,12 +581,11 @@ static cudaError_t w4_launch(const OmegaGpuW4Tensor *t, uint32_t m, const uint16
     if (t->part && (t->fmt || !getenv("B200MOE_W4_FMA"))) {   // tensor-core kernels
         if (m > 16u) return t->fmt == 2 ? w4_rows<2>(t, m, dx, d16, d32, s) : t->fmt ? w4_rows<1>(t, m, dx, d16, d32, s) : w4_rows<0>(t, m, dx, d16, d32, s);
         const dim3 grid(t->n / 128u, 4);
-#define W4_LAUNCH(GQV, FMTV) w4_mma_kernel<GQV, FMTV><<<grid, 512, 16 * (GQV * 64 + 64), s>>>(m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters, nullptr, nullptr, nullptr, nullptr)
+#define W4_LAUNCH(GQV, FMTV) return launch_chained(w4_mma_kernel<GQV, FMTV>, grid, dim3(512), 16 * (GQV * 64 + 64), s, m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters, nullptr, nullptr, nullptr, nullptr)
         if (t->fmt == 2) { if (t->k == 4096u) W4_LAUNCH(32, 2); else if (t->k == 2048u) W4_LAUNCH(16, 2); else if (t->k == 1024u) W4_LAUNCH(8, 2); else W4_LAUNCH(6, 2); }
         else if (t->fmt) { if (t->k == 4096u) W4_LAUNCH(32, 1); else if (t->k == 2048u) W4_LAUNCH(16, 1); else if (t->k == 1024u) W4_LAUNCH(8, 1); else W4_LAUNCH(6, 1); }
         else { if (t->k == 4096u) W4_LAUNCH(32, 0); else if (t->k == 2048u) W4_LAUNCH(16, 0); else if (t->k == 1024u) W4_LAUNCH(8, 0); else W4_LAUNCH(6, 0); }
 #undef W4_LAUNCH
-        return cudaGetLastError();
     }
     const size_t smem = (size_t)W4_MT * t->k * 2;
     static bool attr = false;
