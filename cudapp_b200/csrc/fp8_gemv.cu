@@ -40,6 +40,7 @@ constexpr uint32_t ROWS_WARPS = 4;
 template <int MT> constexpr uint32_t ROWS_CHUNK = MT == 8 ? 2048u : 4096u;   // columns of x resident at a time: at most 64 KB, so that three CTAs share an SM
 template <int LB, int R, int MT>
 __global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? 5 : 3) fp8_rows_kernel(const __grid_constant__ GemvArgs a) {
+    griddep_chain();
     constexpr uint32_t STEP = 32u * LB, CS = ROWS_CHUNK<MT> / STEP, Q = LB / 4, NT = 32u * ROWS_WARPS;
     constexpr int PF = R == 1 ? 4 : 2, PAIRS = R > 1 ? R / 2 : 1;
     using WT = typename WVec<LB>::T;
@@ -76,9 +77,9 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? 5 : 3) fp8_rows_ker
                     v[m] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if ((uint32_t)m >= mc) continue;
                     if (a.x_bf16) {
-                        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(s_row[m] + (size_t)(first + c) * 2));
+                        const uint2 u = *reinterpret_cast<const uint2 *>(s_row[m] + (size_t)(first + c) * 2);
                         v[m] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
-                    } else v[m] = __ldg(reinterpret_cast<const float4 *>(s_row[m] + (size_t)(first + c) * 4));
+                    } else v[m] = *reinterpret_cast<const float4 *>(s_row[m] + (size_t)(first + c) * 4);
                 }
                 const uint32_t st = c / STEP, rem = c % STEP;
                 float4 *to = xs + (size_t)st * MT * Q * 32u + xs_at<LB>((rem % LB) / 4u, rem / LB);
@@ -184,8 +185,7 @@ static cudaError_t launch_one(const GemvArgs &a, dim3 grid, cudaStream_t s) {
     const size_t smem = (size_t)MT * (a.k < ROWS_CHUNK<MT> ? a.k : ROWS_CHUNK<MT>) * 4;
     static const cudaError_t attr = cudaFuncSetAttribute(fp8_rows_kernel<LB, R, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MT * ROWS_CHUNK<MT> * 4));
     if (attr != cudaSuccess) return attr;
-    fp8_rows_kernel<LB, R, MT><<<grid, 32 * ROWS_WARPS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(fp8_rows_kernel<LB, R, MT>, grid, dim3(32 * ROWS_WARPS), smem, s, a);
 }
 template <int R, int MT>
 static cudaError_t launch_lb(const GemvArgs &a, dim3 grid, cudaStream_t s) {
