@@ -35,7 +35,7 @@ struct OmegaGpuW4Tensor {
     uint32_t n, k; uint8_t *w; uint16_t *s;   // s: fp16 scales (int4 format) or, viewed as bytes, E8M0 scales (MXFP4 format)
     uint32_t fmt;                              // 0: signed int4 + fp16 scale per 32; 1: MXFP4 = E2M1 + E8M0 scale per 32
     float *part; uint32_t *counters;   // scratch of the tensor-core kernel: K-quarter partial sums [4][16][n] f32 and one arrival counter per 128 output rows
-    float *gpart; uint32_t *gcounters; uint32_t gtiles, gn;   // the same for the grouped form: per row tile [4][16][gn]; set by omega_gpu_w4_reserve_grouped
+    uint32_t gtiles, gn;   // grouped form: most row tiles of a call, weight rows per expert; set by omega_gpu_w4_reserve_grouped
 };
 
 namespace b200 {
@@ -173,7 +173,7 @@ struct FfnLaunch {
     const unsigned long long *gate, *gate_base; const uint64_t *out_peers, *ret_counters; uint32_t rows_per_rank, ret_index;   // expert parallelism, as in MmaLaunch
     uint32_t wait_limit;
 };
-// grouped 4-bit GEMM over a plan's 16-row tiles (the tensor must have been given its per-tile scratch by omega_gpu_w4_reserve_grouped)
+// grouped 4-bit GEMM over a plan's 16-row tiles (the tensor must have been given its shape by omega_gpu_w4_reserve_grouped)
 cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *x_bf16, uint16_t *y_bf16, float *y_f32, cudaStream_t s);
 bool ffn_shape_ok(uint32_t hidden, uint32_t inter);

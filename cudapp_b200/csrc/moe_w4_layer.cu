@@ -36,7 +36,7 @@ int omega_gpu_moe_w4_layer_create(OmegaGpuW4Tensor *gate_up, OmegaGpuW4Tensor *d
     L->gu = gate_up; L->dn = down; L->experts = experts; L->hidden = H; L->inter = I; L->topk = topk; L->max_tokens = max_tokens; L->norm_topk = norm_topk;
     const size_t T = max_tokens, R = T * topk;
     L->max_tiles = (uint32_t)(R / 16 + experts + 8);
-    // the per-tile scratch of the two grouped GEMMs (each call takes the library's lock itself)
+    // the shapes of the two grouped GEMMs (each call takes the library's lock itself)
     int rc = omega_gpu_w4_reserve_grouped(gate_up, 2u * I, L->max_tiles);
     if (rc == OMEGA_GPU_FP8_OK) rc = omega_gpu_w4_reserve_grouped(down, H, L->max_tiles);
     if (rc != OMEGA_GPU_FP8_OK) { free(L); return rc; }

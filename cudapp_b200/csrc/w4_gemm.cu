@@ -2,8 +2,8 @@
 // columns) times bf16 activations, f32 accumulation, bf16 output. The reference has no integer-W4 arithmetic
 // (docs/models/QUANT.md:62 of the reference: "integer W4 refuses"), so this follows the benchmark definition only:
 // y[m][r] = sum over groups g of scale[r][g] * sum_{c in g} x[m][c] * q[r][c].
-// Three kernels. The tensor-core kernels take the shapes they are written for (n a multiple of 128; k 768, 1024, 2048 or 4096), one up to 16 rows (and a routing plan's tiles), the
-// other more; the CUDA-core kernel takes every other shape: a warp owns RW output rows; lane l owns K groups l, l+32, ... (16 contiguous bytes
+// Three kernels. The tensor-core kernels take the shapes they are written for (n a multiple of 128; k 768, 1024, 2048 or 4096), one up to 16 rows, the
+// other more (and a routing plan's tiles); the CUDA-core kernel takes every other shape: a warp owns RW output rows; lane l owns K groups l, l+32, ... (16 contiguous bytes
 // each, 512 contiguous bytes per warp load); the activation panel sits in shared memory as bf16.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -133,23 +133,11 @@ __device__ __forceinline__ float ue4m3_f32(uint32_t c) { return (c >> 3) ? __uin
 // the words of quad threads t/2 and 2 + t/2 (one shuffle each); each MMA goes into its own fresh accumulator and is scaled by its own scale.
 template <int GQ, int FMT>   // 32-column groups per K quarter: k = 128 * GQ; FMT 0: int4 + fp16 scales, 1: E2M1 + E8M0 scales (MXFP4), 2: E2M1 + UE4M3 per 16 (NVFP4)
 __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint16_t *__restrict__ sc,
-                                                        const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32, float *part, uint32_t *counters,
-                                                        const uint4 *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap) {
+                                                        const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32, float *part, uint32_t *counters) {
     constexpr uint32_t KQ = GQ * 32u, XS = KQ * 2u + 64u;   // columns per quarter; bytes between panel rows (the 64 keep a quarter-warp's 16-byte reads on separate banks)
     extern __shared__ __align__(16) uint8_t xq[];
     __shared__ uint32_t s_last;
     const uint32_t nb = blockIdx.x, kq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, t = lane & 3u;
-    // grouped form (tiles != null): blockIdx.z is a row tile {expert, first sorted row, rows <= 16} of a routing plan; the tensor holds the experts' matrices
-    // one after the other (n rows each); activation row i of the tile is x[xmap[row0 + i]] (or row0 + i), its result goes to row ymap[row0 + i] (or row0 + i)
-    uint32_t mt = 0, row0 = 0;
-    if (tiles) {
-        griddep_chain();
-        if (blockIdx.z >= header[2]) return;
-        const uint4 tl = tiles[blockIdx.z];
-        w += (size_t)tl.x * n * (k / 2u); sc = reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(sc) + (size_t)tl.x * n * (k / 32u) * (FMT == 1 ? 1u : 2u));
-        row0 = tl.y; mt = min(16u, tl.z);
-        part += (size_t)blockIdx.z * 4u * 16u * n; counters += (size_t)blockIdx.z * (n / 128u);
-    } else mt = m;
     // this thread's weight words: output row n0 + r, word t of every group of the quarter; all requested before anything else
     const uint32_t n0 = nb * 128u + warp * 8u;
     const uint32_t *wrow = reinterpret_cast<const uint32_t *>(w + (size_t)(n0 + r) * (k / 2u) + (size_t)kq * (KQ / 2u));
@@ -175,12 +163,12 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
             reinterpret_cast<uint16_t *>(&sv1[0])[i] = __ldg(reinterpret_cast<const uint16_t *>(s1b) + i);
         }
     }
-    if (!tiles) griddep_chain();   // the weights are the tensor's own: only what follows depends on earlier work
+    griddep_chain();   // the weights are the tensor's own: only what follows depends on earlier work
     // the quarter of the activation panel: 16 rows (zero past the last), columns kq * KQ ..
     for (uint32_t i = threadIdx.x; i < 16u * (KQ / 8u); i += 512u) {
         const uint32_t row = i / (KQ / 8u), c8 = i - row * (KQ / 8u);
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < mt) v = reinterpret_cast<const uint4 *>(x + (size_t)(xmap ? xmap[row0 + row] : row0 + row) * k + (size_t)kq * KQ)[c8];
+        if (row < m) v = reinterpret_cast<const uint4 *>(x + (size_t)row * k + (size_t)kq * KQ)[c8];
         *reinterpret_cast<uint4 *>(xq + row * XS + c8 * 16u) = v;
     }
     __syncthreads();
@@ -233,11 +221,11 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
     __threadfence();
     for (uint32_t i = threadIdx.x; i < 16u * 128u; i += 512u) {
         const uint32_t row = i >> 7, col = nb * 128u + (i & 127u);
-        if (row >= mt) continue;
+        if (row >= m) continue;
         float v = __ldcg(part + (size_t)row * n + col);
 #pragma unroll
         for (uint32_t q = 1; q < 4; q++) v = __fadd_rn(v, __ldcg(part + ((size_t)q * 16u + row) * n + col));
-        const size_t at = (size_t)(ymap ? ymap[row0 + row] : row0 + row) * n + col;
+        const size_t at = (size_t)row * n + col;
         if (y32) y32[at] = v;
         if (y16) { const uint32_t b = __float_as_uint(v); y16[at] = (uint16_t)(((b & 0x7fffffffu) > 0x7f800000u) ? ((b >> 16) | 0x40u) : ((b + 0x7fffu + ((b >> 16) & 1u)) >> 16)); }
     }
@@ -267,28 +255,43 @@ __device__ __forceinline__ void mma_bf16_add(float *d, uint32_t a0, uint32_t a1,
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __host__ __device__ constexpr uint32_t w4_rows_stage(int MT, int NT) { return MT * 8192u + NT * 2048u + NT * 256u; }   // bytes: x, weights, scales of one step
-constexpr uint32_t w4_rows_smem(int MT, int NT) {
-    const uint32_t red = 4u * MT * 16u * (16u * NT + 8u) * 4u, st = 2u * w4_rows_stage(MT, NT);     // the quarters' sums reuse the stages
+constexpr uint32_t w4_rows_smem(int MT, int NT, int ST) {
+    const uint32_t red = 4u * MT * 16u * (16u * NT + 8u) * 4u, st = (uint32_t)ST * w4_rows_stage(MT, NT);     // the quarters' sums reuse the stages
     return red > st ? red : st;
 }
 
-template <int FMT, int MT, int NT>
-__global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint8_t *__restrict__ sc,
-                                                             const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32) {
+// Grouped form (GROUPED, MT = 1): a CTA's rows are a row tile {expert, first sorted row, rows <= 16} of a routing plan; the tensor holds the experts' matrices one
+// after the other (n rows each); activation row i of the tile is x[xmap[row0 + i]] (or row0 + i), its result goes to row ymap[row0 + i] (or row0 + i).
+struct W4Group { const uint4 *tiles; const uint32_t *header, *xmap, *ymap; };
+
+template <int FMT, int MT, int NT, int ST, bool GROUPED>
+__global__ void __launch_bounds__(256, GROUPED ? 4 : 2) w4_mma_rows_kernel(uint32_t m, uint32_t n, uint32_t k, const uint8_t *__restrict__ w, const uint8_t *__restrict__ sc,
+                                                             const uint16_t *x, uint16_t *__restrict__ y16, float *__restrict__ y32, const W4Group grp) {
+    static_assert(!GROUPED || MT == 1, "a plan's tile has at most 16 rows");
     griddep_chain();
     constexpr uint32_t ROWS = MT * 16u, COLS = NT * 16u, WOFF = MT * 8192u, SOFF = WOFF + NT * 2048u, STAGE = w4_rows_stage(MT, NT), RS = COLS + 8u;
     constexpr uint32_t SB = FMT == 1 ? 1u : 2u;   // scale bytes per 32 columns
     extern __shared__ __align__(16) uint8_t sm[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, t = lane & 3u, kq = warp >> 1, half = warp & 1u;
-    const uint32_t ct = n / COLS, m0 = blockIdx.x / ct * ROWS, n0 = blockIdx.x % ct * COLS, GQ = k / 128u, steps = GQ / 2u, srow = k / 32u * SB;
+    const uint32_t ct = n / COLS, tile = blockIdx.x / ct, n0 = blockIdx.x % ct * COLS, GQ = k / 128u, steps = GQ / 2u, srow = k / 32u * SB;
+    uint32_t m0 = tile * ROWS;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+    const uint16_t *x0 = nullptr;   // grouped: this thread's row of the tile
+    if (GROUPED) {
+        if (tile >= grp.header[2]) return;
+        const uint4 tl = grp.tiles[tile];
+        w += (size_t)tl.x * n * (k / 2u); sc += (size_t)tl.x * n * srow;
+        m0 = tl.y; m = m0 + min(16u, tl.z);
+        const uint32_t row = m0 + (threadIdx.x >> 3), from = row < m ? row : m0;
+        x0 = x + (size_t)(grp.xmap ? grp.xmap[from] : from) * k;
+    }
     auto load = [&](uint32_t step, uint32_t st) {
         const uint32_t b = base + st * STAGE;
 #pragma unroll 1
         for (uint32_t row = threadIdx.x >> 3; row < ROWS; row += 32u) {   // not unrolled: the addresses would take the registers of the sums
             const uint32_t c = threadIdx.x & 7u, dst = b + row * 128u + w4_chunk(row, c) * 16u;
             const bool in = m0 + row < m;
-            const uint16_t *src = x + (size_t)(in ? m0 + row : m0) * k + step * 64u + c * 8u;
+            const uint16_t *src = (GROUPED ? x0 : x + (size_t)(in ? m0 + row : m0) * k) + step * 64u + c * 8u;
 #pragma unroll
             for (uint32_t q = 0; q < 4; q++) cp16(dst + q * ROWS * 128u, src + q * (k / 4u), in ? 16u : 0u);
         }
@@ -297,23 +300,26 @@ __global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_
             const uint32_t q = i / (2u * COLS), col = (i >> 1) % COLS, g = i & 1u;
             cp16(b + WOFF + ((q * 2u + g) * COLS + col) * 16u, w + (size_t)(n0 + col) * (k / 2u) + q * (k / 8u) + (step * 2u + g) * 16u, 16u);
         }
-        if (threadIdx.x < 4u * COLS) {   // one byte per group: the aligned word that holds this step's two
-            const uint32_t q = threadIdx.x / COLS, col = threadIdx.x % COLS;
-            cp4(b + SOFF + threadIdx.x * 4u, sc + (size_t)(n0 + col) * srow + ((q * GQ + step * 2u) * SB & ~3u));
+        for (uint32_t i = threadIdx.x; i < 4u * COLS; i += 256u) {   // FMT 1 has one byte per group: the aligned word that holds this step's two
+            const uint32_t q = i / COLS, col = i % COLS;
+            cp4(b + SOFF + i * 4u, sc + (size_t)(n0 + col) * srow + ((q * GQ + step * 2u) * SB & ~3u));
         }
-        asm volatile("cp.async.commit_group;");
     };
+    auto commit = [] { asm volatile("cp.async.commit_group;"); };
     float acc[MT][NT][4];
 #pragma unroll
     for (int i = 0; i < MT; i++)
 #pragma unroll
         for (int j = 0; j < NT; j++) { acc[i][j][0] = 0.0f; acc[i][j][1] = 0.0f; acc[i][j][2] = 0.0f; acc[i][j][3] = 0.0f; }
-    load(0, 0);
+#pragma unroll
+    for (uint32_t p = 0; p < ST - 1u; p++) { if (p < steps) load(p, p); commit(); }
+    uint32_t st = 0;
     for (uint32_t step = 0; step < steps; step++) {
-        if (step + 1u < steps) { load(step + 1u, (step + 1u) & 1u); asm volatile("cp.async.wait_group 1;"); }
-        else asm volatile("cp.async.wait_group 0;");
-        __syncthreads();
-        const uint8_t *b = sm + (step & 1u) * STAGE, *xs = b + kq * ROWS * 128u;
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");   // this step's stage has arrived
+        __syncthreads();                                                    // ... for every thread, and the stage of the step before is free
+        if (step + ST - 1u < steps) load(step + ST - 1u, st ? st - 1u : ST - 1u);
+        commit();
+        const uint8_t *b = sm + st * STAGE, *xs = b + kq * ROWS * 128u;
         const uint32_t *ws = reinterpret_cast<const uint32_t *>(b + WOFF) + (kq * 2u * COLS + half * 8u * NT) * 4u;
         const uint32_t *ss = reinterpret_cast<const uint32_t *>(b + SOFF) + kq * COLS + half * 8u * NT;
 #pragma unroll
@@ -367,8 +373,9 @@ __global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_
                 }
             }
         }
-        __syncthreads();
+        st = st + 1u == ST ? 0u : st + 1u;
     }
+    __syncthreads();
     float *red = reinterpret_cast<float *>(sm);   // [quarter][row][RS]
 #pragma unroll
     for (int i = 0; i < MT; i++)
@@ -385,19 +392,19 @@ __global__ void __launch_bounds__(256, 2) w4_mma_rows_kernel(uint32_t m, uint32_
         float v = red[row * RS + col];
 #pragma unroll
         for (uint32_t q = 1; q < 4; q++) v = __fadd_rn(v, red[(q * ROWS + row) * RS + col]);
-        const size_t at = (size_t)(m0 + row) * n + n0 + col;
+        const size_t at = (size_t)(GROUPED && grp.ymap ? grp.ymap[m0 + row] : m0 + row) * n + n0 + col;
         if (y32) y32[at] = v;
         if (y16) { const uint32_t u = __float_as_uint(v); y16[at] = (uint16_t)(((u & 0x7fffffffu) > 0x7f800000u) ? ((u >> 16) | 0x40u) : ((u + 0x7fffu + ((u >> 16) & 1u)) >> 16)); }
     }
 }
 
-template <int FMT, int MT, int NT>
-static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
+template <int FMT, int MT, int NT, int ST, bool GROUPED>
+static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, uint32_t n, uint32_t tiles, const uint16_t *dx, uint16_t *d16, float *d32, const W4Group &grp, cudaStream_t s) {
     // set on every call: it belongs to the device's context and costs well under a launch
-    const cudaError_t e = cudaFuncSetAttribute(w4_mma_rows_kernel<FMT, MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4_rows_smem(MT, NT));
+    const cudaError_t e = cudaFuncSetAttribute(w4_mma_rows_kernel<FMT, MT, NT, ST, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4_rows_smem(MT, NT, ST));
     if (e != cudaSuccess) return e;
-    return launch_chained(w4_mma_rows_kernel<FMT, MT, NT>, dim3(t->n / (16u * NT) * ((m + 16u * MT - 1u) / (16u * MT))), dim3(256), w4_rows_smem(MT, NT), s,
-                          m, t->n, t->k, t->w, reinterpret_cast<const uint8_t *>(t->s), dx, d16, d32);
+    return launch_chained(w4_mma_rows_kernel<FMT, MT, NT, ST, GROUPED>, dim3(n / (16u * NT) * tiles), dim3(256), w4_rows_smem(MT, NT, ST), s,
+                          m, n, t->k, t->w, reinterpret_cast<const uint8_t *>(t->s), dx, d16, d32, grp);
 }
 template <int FMT>
 static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
@@ -412,11 +419,11 @@ static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t
         if (v < cost) { cost = v; best = c; }
     }
     switch (best) {
-    case 0: return w4_rows_start<FMT, 2, 4>(t, m, dx, d16, d32, s);
-    case 1: return w4_rows_start<FMT, 3, 4>(t, m, dx, d16, d32, s);
-    case 2: return w4_rows_start<FMT, 4, 4>(t, m, dx, d16, d32, s);
-    case 3: return w4_rows_start<FMT, 5, 4>(t, m, dx, d16, d32, s);
-    default: return w4_rows_start<FMT, 2, 2>(t, m, dx, d16, d32, s);
+    case 0: return w4_rows_start<FMT, 2, 4, 2, false>(t, m, t->n, (tiles + 1u) / 2u, dx, d16, d32, W4Group(), s);
+    case 1: return w4_rows_start<FMT, 3, 4, 2, false>(t, m, t->n, (tiles + 2u) / 3u, dx, d16, d32, W4Group(), s);
+    case 2: return w4_rows_start<FMT, 4, 4, 2, false>(t, m, t->n, (tiles + 3u) / 4u, dx, d16, d32, W4Group(), s);
+    case 3: return w4_rows_start<FMT, 5, 4, 2, false>(t, m, t->n, (tiles + 4u) / 5u, dx, d16, d32, W4Group(), s);
+    default: return w4_rows_start<FMT, 2, 2, 2, false>(t, m, t->n, (tiles + 1u) / 2u, dx, d16, d32, W4Group(), s);
     }
 }
 
@@ -460,15 +467,16 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
     scales[b] = (uint8_t)sc;
 }
 
+template <int FMT>
+static cudaError_t w4_grouped(const OmegaGpuW4Tensor *t, const W4Group &grp, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
+    // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often and were slower (64-token MXFP4 layer:
+    // 279 us, 274 with 64 columns, 307 with 128; 64-token int4 layer of 32 experts, hidden 4096: 178, 188 and 203 us).
+    return w4_rows_start<FMT, 1, 2, 4, true>(t, 0, t->gn, t->gtiles, dx, d16, d32, grp, s);
+}
 cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
-    const dim3 grid(t->gn / 128u, 4, t->gtiles);
-#define W4_GROUPED(GQV, FMTV) return launch_chained(w4_mma_kernel<GQV, FMTV>, grid, dim3(512), 16 * (GQV * 64 + 64), s, 0u, t->gn, t->k, t->w, t->s, dx, d16, d32, t->gpart, \
-        t->gcounters, (const uint4 *)tiles, header, xmap, ymap)
-    if (t->fmt == 2) { if (t->k == 4096u) W4_GROUPED(32, 2); else if (t->k == 2048u) W4_GROUPED(16, 2); else if (t->k == 1024u) W4_GROUPED(8, 2); else W4_GROUPED(6, 2); }
-    else if (t->fmt) { if (t->k == 4096u) W4_GROUPED(32, 1); else if (t->k == 2048u) W4_GROUPED(16, 1); else if (t->k == 1024u) W4_GROUPED(8, 1); else W4_GROUPED(6, 1); }
-    else { if (t->k == 4096u) W4_GROUPED(32, 0); else if (t->k == 2048u) W4_GROUPED(16, 0); else if (t->k == 1024u) W4_GROUPED(8, 0); else W4_GROUPED(6, 0); }
-#undef W4_GROUPED
+    const W4Group grp = {(const uint4 *)tiles, header, xmap, ymap};
+    return t->fmt == 2 ? w4_grouped<2>(t, grp, dx, d16, d32, s) : t->fmt ? w4_grouped<1>(t, grp, dx, d16, d32, s) : w4_grouped<0>(t, grp, dx, d16, d32, s);
 }
 
 }  // namespace b200
@@ -573,15 +581,13 @@ void omega_gpu_w4_free(OmegaGpuW4Tensor *t) {
     if (t->s) cudaFree(t->s);
     if (t->part) cudaFree(t->part);
     if (t->counters) cudaFree(t->counters);
-    if (t->gpart) cudaFree(t->gpart);
-    if (t->gcounters) cudaFree(t->gcounters);
     free(t);
 }
 static cudaError_t w4_launch(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     if (t->part && (t->fmt || !getenv("B200MOE_W4_FMA"))) {   // tensor-core kernels
         if (m > 16u) return t->fmt == 2 ? w4_rows<2>(t, m, dx, d16, d32, s) : t->fmt ? w4_rows<1>(t, m, dx, d16, d32, s) : w4_rows<0>(t, m, dx, d16, d32, s);
         const dim3 grid(t->n / 128u, 4);
-#define W4_LAUNCH(GQV, FMTV) return launch_chained(w4_mma_kernel<GQV, FMTV>, grid, dim3(512), 16 * (GQV * 64 + 64), s, m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters, nullptr, nullptr, nullptr, nullptr)
+#define W4_LAUNCH(GQV, FMTV) return launch_chained(w4_mma_kernel<GQV, FMTV>, grid, dim3(512), 16 * (GQV * 64 + 64), s, m, t->n, t->k, t->w, t->s, dx, d16, d32, t->part, t->counters)
         if (t->fmt == 2) { if (t->k == 4096u) W4_LAUNCH(32, 2); else if (t->k == 2048u) W4_LAUNCH(16, 2); else if (t->k == 1024u) W4_LAUNCH(8, 2); else W4_LAUNCH(6, 2); }
         else if (t->fmt) { if (t->k == 4096u) W4_LAUNCH(32, 1); else if (t->k == 2048u) W4_LAUNCH(16, 1); else if (t->k == 1024u) W4_LAUNCH(8, 1); else W4_LAUNCH(6, 1); }
         else { if (t->k == 4096u) W4_LAUNCH(32, 0); else if (t->k == 2048u) W4_LAUNCH(16, 0); else if (t->k == 1024u) W4_LAUNCH(8, 0); else W4_LAUNCH(6, 0); }
@@ -596,24 +602,18 @@ static cudaError_t w4_launch(const OmegaGpuW4Tensor *t, uint32_t m, const uint16
 }
 /* Grouped form: the tensor holds `experts` matrices of n_per_expert rows one after the other (uploaded as one tensor of experts x n_per_expert rows);
  * the rows to multiply come sorted by expert with a tile table of a routing plan made with tile_rows = 16 (omega_gpu_moe_plan_async: tiles {expert, first
- * row, rows}, header[2] = tiles). reserve allocates the per-tile scratch once (blocking); the async entry queues one launch and allocates nothing. */
+ * row, rows}, header[2] = tiles). reserve sets the shape and the most tiles of a call; the async entry queues one launch and allocates nothing. */
 int omega_gpu_w4_reserve_grouped(OmegaGpuW4Tensor *t, uint32_t n_per_expert, uint32_t max_tiles) {
     if (!t || !n_per_expert || !max_tiles || n_per_expert % 128u || t->n % n_per_expert || !(t->k == 768u || t->k == 1024u || t->k == 2048u || t->k == 4096u)) return OMEGA_GPU_FP8_BAD_ARGS;
     Lock l;
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
-    if (t->gpart) { cudaFree(t->gpart); t->gpart = nullptr; }
-    if (t->gcounters) { cudaFree(t->gcounters); t->gcounters = nullptr; }
-    const size_t pb = (size_t)max_tiles * 4 * 16 * n_per_expert * 4, cb = (size_t)max_tiles * (n_per_expert / 128u) * 4;
-    const bool ok = cuda_ok(cudaMalloc(&t->gpart, pb), "cudaMalloc(w4 grouped partials)") && cuda_ok(cudaMalloc(&t->gcounters, cb), "cudaMalloc(w4 grouped counters)") &&
-                    cuda_ok(cudaMemset(t->gcounters, 0, cb), "memset");
-    if (!ok) { if (t->gpart) cudaFree(t->gpart); if (t->gcounters) cudaFree(t->gcounters); t->gpart = nullptr; t->gcounters = nullptr; return OMEGA_GPU_FP8_CHIP_FAIL; }
     t->gtiles = max_tiles; t->gn = n_per_expert;
     return OMEGA_GPU_FP8_OK;
 }
 int omega_gpu_w4_gemm_grouped_async(const OmegaGpuW4Tensor *t, uint64_t tiles_va, uint64_t header_va, uint64_t xmap_va, uint64_t ymap_va,
                                     uint64_t x_bf16_va, uint64_t y_bf16_va, uint64_t y_f32_va, void *stream) {
     if (!t || !tiles_va || !header_va || !x_bf16_va || (!y_bf16_va && !y_f32_va)) return OMEGA_GPU_FP8_BAD_ARGS;
-    if (!t->gpart || !t->gtiles) { set_error("w4 grouped gemm: call omega_gpu_w4_reserve_grouped first"); return OMEGA_GPU_FP8_BAD_ARGS; }
+    if (!t->gtiles) { set_error("w4 grouped gemm: call omega_gpu_w4_reserve_grouped first"); return OMEGA_GPU_FP8_BAD_ARGS; }
     if (!st().opened || st().latched) return OMEGA_GPU_FP8_CHIP_FAIL;
     return cuda_ok(launch_w4_grouped(t, (const void *)(uintptr_t)tiles_va, (const uint32_t *)(uintptr_t)header_va, (const uint32_t *)(uintptr_t)xmap_va, (const uint32_t *)(uintptr_t)ymap_va,
                                      (const uint16_t *)(uintptr_t)x_bf16_va, (uint16_t *)(uintptr_t)y_bf16_va, (float *)(uintptr_t)y_f32_va, (cudaStream_t)stream), "w4 grouped launch")
