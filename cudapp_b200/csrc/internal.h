@@ -132,6 +132,10 @@ cudaError_t launch_topk(uint32_t tokens, uint32_t experts, uint32_t topk, int no
 cudaError_t launch_plan(uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows, const uint32_t *ids,
                         const OmegaGpuMoePlanOut &o, cudaStream_t s, uint32_t *scratch = nullptr, size_t scratch_words = 0);
 size_t plan_scratch_words(uint32_t picks, uint32_t experts);
+// top-k and plan in one launch, where route_ok: routed = columns of the logits, experts = those plus a shared one, slots as in launch_topk
+bool route_ok(uint32_t tokens, uint32_t routed, uint32_t experts);
+cudaError_t launch_route(uint32_t tokens, uint32_t routed, uint32_t topk, int norm, uint32_t slots, uint32_t experts, uint32_t tile_rows, const uint16_t *logits, uint32_t *ids, float *wts,
+                         const OmegaGpuMoePlanOut &o, cudaStream_t s);
 uint32_t plan_launch_count(uint32_t picks, uint32_t experts, const uint32_t *scratch, size_t scratch_words, const OmegaGpuMoePlanOut &o);
 // routing plans of several layers in one launch (one CTA per layer); element strides between layers
 struct PlanBatch { uint32_t *counts, *starts, *xmap, *ymap, *pos, *header; uint4 *tiles; size_t map_stride, tile_stride; };

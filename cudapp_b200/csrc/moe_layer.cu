@@ -91,11 +91,12 @@ bool layer_forward(OmegaGpuMoeLayer *L, uint32_t tokens, const uint16_t *logits,
     uint32_t n = 0;
 #define MARK(name) do { L->names[n] = name; if (L->prof) cudaEventRecord(L->prof[n + 1], s); n++; } while (0)
     if (L->prof) cudaEventRecord(L->prof[0], s);
+    const bool one_route = !ids_in && route_ok(tokens, E - L->shared, E);
     if (ids_in) {
         if (!cuda_ok(cudaMemcpyAsync(w->ids, ids_in, (size_t)R * 4, cudaMemcpyDeviceToDevice, s), "copy ids") ||
             !cuda_ok(cudaMemcpyAsync(w->wts, wts_in, (size_t)R * 4, cudaMemcpyDeviceToDevice, s), "copy weights")) return false;
         MARK("routing_copy");
-    } else {
+    } else if (!one_route) {
         if (!cuda_ok(launch_topk(tokens, E - L->shared, L->routed_topk, (int)L->cfg.norm_topk, logits, w->ids, w->wts, s, K), "topk launch")) return false;
         MARK("topk");
     }
@@ -108,9 +109,15 @@ bool layer_forward(OmegaGpuMoeLayer *L, uint32_t tokens, const uint16_t *logits,
     // prefill-sized segments (64 rows per expert on average, or on request) take the 128-row-tile kernel
     const bool wide = mma && L->wide_ok && (L->cfg.tile_rows == 128u || (L->cfg.tile_rows == 0u && R >= 64u * E));
     o.tiles_va = mma ? (uint64_t)(uintptr_t)w->tiles : 0;
-    if (!cuda_ok(launch_plan(tokens, K, E, K, mma ? (wide ? mma_wide_tile_rows() : L->tile_rows) : 0, w->ids, o, s, w->plan_scratch, w->plan_scratch_words), "plan launch")) return false;
-    MARK("plan");
-    const uint32_t extra = plan_launch_count(R, E, w->plan_scratch, w->plan_scratch_words, o) - 1u;   // launches behind that one mark
+    const uint32_t tile_rows = mma ? (wide ? mma_wide_tile_rows() : L->tile_rows) : 0;
+    if (one_route) {
+        if (!cuda_ok(launch_route(tokens, E - L->shared, L->routed_topk, (int)L->cfg.norm_topk, K, E, tile_rows, logits, w->ids, w->wts, o, s), "route launch")) return false;
+        MARK("topk_plan");
+    } else {
+        if (!cuda_ok(launch_plan(tokens, K, E, K, tile_rows, w->ids, o, s, w->plan_scratch, w->plan_scratch_words), "plan launch")) return false;
+        MARK("plan");
+    }
+    const uint32_t extra = one_route ? 0u : plan_launch_count(R, E, w->plan_scratch, w->plan_scratch_words, o) - 1u;   // launches behind that one mark
     if (mma) {
         // activations as e4m3 pieces in sorted-row order, then the two tensor-core grouped GEMMs
         const uint32_t Px = L->cfg.x_pieces, Pa = L->cfg.act_pieces, Rp = w->max_tokens * w->topk + 8;

@@ -163,6 +163,31 @@ __global__ void __launch_bounds__(1024) plan_kernel(uint32_t tokens, uint32_t sl
     griddep_chain();
     plan_body(tokens, slots, experts, ystride, tile_rows, ids, o, nullptr);
 }
+// Top-k and plan of at most 32 tokens in one launch: the plan is one CTA of 32 warps anyway, and a warp per token makes the picks first. Both parts are
+// latency, so what the second launch cost (its gap, and the picks' way through L2) is what is saved: one-token layer 39.7 -> 39.0 us. Past 32 tokens a warp would make
+// several tokens' picks in turn.
+// dynamic shared: what plan_body needs, then the tokens' logits as f32
+static size_t plan_smem(uint32_t experts) { return (size_t)experts * 12 + 96 * 4 + (size_t)32 * experts * 2; }
+__global__ void __launch_bounds__(1024) route_kernel(uint32_t tokens, uint32_t routed, uint32_t topk, int norm, uint32_t slots, uint32_t experts, uint32_t tile_rows,
+                                                     const uint16_t *logits, uint32_t *ids, float *wts, const OmegaGpuMoePlanOut o) {
+    griddep_chain();
+    extern __shared__ uint32_t smem[];
+    const uint32_t lane = threadIdx.x & 31u, t = threadIdx.x >> 5;
+    if (t < tokens) {
+        float *l = reinterpret_cast<float *>(smem + 19u * experts + 96u) + (size_t)t * routed;
+        for (uint32_t e = lane; e < routed; e += 32) l[e] = __uint_as_float((uint32_t)logits[(size_t)t * routed + e] << 16);
+        __syncwarp();
+        warp_topk(l, routed, topk, norm, ids + (size_t)t * slots, wts + (size_t)t * slots);
+        if (slots > topk && lane == 0) { ids[(size_t)t * slots + topk] = routed; wts[(size_t)t * slots + topk] = 1.0f; }
+    }
+    __syncthreads();
+    plan_body(tokens, slots, experts, slots, tile_rows, ids, o, nullptr);
+}
+bool route_ok(uint32_t tokens, uint32_t routed, uint32_t experts) { return tokens <= 32u && plan_smem(experts) + (size_t)tokens * routed * 4 <= 48 * 1024; }
+cudaError_t launch_route(uint32_t tokens, uint32_t routed, uint32_t topk, int norm, uint32_t slots, uint32_t experts, uint32_t tile_rows, const uint16_t *logits, uint32_t *ids, float *wts,
+                         const OmegaGpuMoePlanOut &o, cudaStream_t s) {
+    return launch_chained(route_kernel, dim3(1), dim3(1024), plan_smem(experts) + (size_t)tokens * routed * 4, s, tokens, routed, topk, norm, slots, experts, tile_rows, logits, ids, wts, o);
+}
 // one CTA per layer: layer l's picks at ids + l * tokens * slots, its outputs at the PlanBatch strides
 __global__ void __launch_bounds__(1024) plan_batch_kernel(uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows,
                                                           const uint32_t *ids, const PlanBatch b) {
@@ -176,7 +201,7 @@ __global__ void __launch_bounds__(1024) plan_batch_kernel(uint32_t tokens, uint3
 }
 cudaError_t launch_plan_batch(uint32_t layers, uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t ystride, uint32_t tile_rows, const uint32_t *ids,
                               const PlanBatch &b, cudaStream_t s) {
-    const size_t smem = (size_t)experts * 12 + 96 * 4 + (size_t)32 * experts * 2;
+    const size_t smem = plan_smem(experts);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(plan_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -267,7 +292,7 @@ cudaError_t launch_plan(uint32_t tokens, uint32_t slots, uint32_t experts, uint3
         return e;
     }
 
-    const size_t smem = (size_t)experts * 12 + 96 * 4 + (size_t)32 * experts * 2;
+    const size_t smem = plan_smem(experts);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
