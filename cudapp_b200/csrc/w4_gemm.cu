@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
 // quarter. A step is two scale groups of every quarter: rows of x (64 columns), weights (two 16-byte groups a row) and scales (4 bytes a row) come by
 // cp.async into one of two stages while the other is used. Two CTAs per SM (128 registers). The 16-byte chunks of a row of x are permuted by
 // bits 0 and 1 of the row, so that a quad's fragments of neighbouring rows fall on different banks.
-// Measured with a cold L2 against launches of 16 rows (int4 / MXFP4 / NVFP4): 300 x 4096 x 2048 169 / 171 / 205 -> 49 / 51 / 61 us, 17 x 4096 x 2048
-// 21.5 / 21.5 / 25.6 -> 14.3 us, 512 x 8192 x 4096 698 / 756 / 916 -> 215 / 227 / 270 us.
+// Measured with a cold L2 against launches of 16 rows (int4 / MXFP4 / NVFP4): 300 x 4096 x 2048 169 / 171 / 205 -> 49 / 47 / 57 us, 17 x 4096 x 2048
+// 21.5 / 21.5 / 25.6 -> 14.3 us, 512 x 8192 x 4096 698 / 756 / 916 -> 199 / 215 / 262 us.
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, uint32_t bytes) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)); }
 __device__ __forceinline__ void cp4(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src)); }
 __device__ __forceinline__ uint32_t w4_chunk(uint32_t row, uint32_t c) { return c ^ (((row & 1u) << 2) | (row & 2u)); }
@@ -408,7 +408,7 @@ static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, uint32_t
 template <int FMT>
 static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     // Few CTAs want small tiles, many want tall ones (a decoded weight is used more often); in between the number of waves decides. The cost of a tile is its
-    // MT x NT products, its decoding (NT) and a fixed part. Measured (int4): 17 x 4096 x 2048 14.3 us at 2 x 2 and 26.6 at 4 x 4; 512 x 8192 x 4096 215 us at
+    // MT x NT products, its decoding (NT) and a fixed part. Measured (int4, before the decode by word): 17 x 4096 x 2048 14.3 us at 2 x 2 and 26.6 at 4 x 4; 512 x 8192 x 4096 215 us at
     // 4 x 4 and 268 at 2 x 2; 300 x 4096 x 2048 49 us at 5 x 4 (one wave, although some of its sums spill) and 55 at 4 x 4 (two waves).
     const uint32_t slots = 2u * (uint32_t)(st().sm_count ? st().sm_count : 148), tiles = (m + 15u) / 16u;
     uint32_t best = 0, cost = ~0u;
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
 
 template <int FMT>
 static cudaError_t w4_grouped(const OmegaGpuW4Tensor *t, const W4Group &grp, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
-    // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often and were slower (64-token MXFP4 layer:
+    // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often and were slower (before the decode by word, 64-token MXFP4 layer:
     // 279 us, 274 with 64 columns, 307 with 128; 64-token int4 layer of 32 experts, hidden 4096: 178, 188 and 203 us).
     return w4_rows_start<FMT, 1, 2, 4, true>(t, 0, t->gn, t->gtiles, dx, d16, d32, grp, s);
 }
