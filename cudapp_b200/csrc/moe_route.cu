@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(1024) route_kernel(uint32_t tokens, uint32_t r
     __syncthreads();
     plan_body(tokens, slots, experts, slots, tile_rows, ids, o, nullptr);
 }
-bool route_ok(uint32_t tokens, uint32_t routed, uint32_t experts) { return tokens <= 32u && plan_smem(experts) + (size_t)tokens * routed * 4 <= 48 * 1024; }
+// The launch has to stay within the 48 KB that a block may use without an opt-in, and plan_body's static words count towards them: 64 bytes are left for those.
+bool route_ok(uint32_t tokens, uint32_t routed, uint32_t experts) { return tokens <= 32u && plan_smem(experts) + (size_t)tokens * routed * 4 <= 48 * 1024 - 64; }
 cudaError_t launch_route(uint32_t tokens, uint32_t routed, uint32_t topk, int norm, uint32_t slots, uint32_t experts, uint32_t tile_rows, const uint16_t *logits, uint32_t *ids, float *wts,
                          const OmegaGpuMoePlanOut &o, cudaStream_t s) {
     return launch_chained(route_kernel, dim3(1), dim3(1024), plan_smem(experts) + (size_t)tokens * routed * 4, s, tokens, routed, topk, norm, slots, experts, tile_rows, logits, ids, wts, o);
