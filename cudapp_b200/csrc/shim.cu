@@ -72,13 +72,15 @@ static bool pinned_open() {
     return true;
 }
 void *result_area() { return pinned_open() ? st().pinned + RING * RING_CHUNK : nullptr; }
-bool host_pinned(const void *p) {
+// memory that the driver does not know: plain pageable host memory. Only that may be touched by the host here; everything else, a device or managed
+// address among it (the entries have always taken those), goes to the driver's copy as it is.
+static bool pageable(const void *p) {
     cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { (void)cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { (void)cudaGetLastError(); return true; }
+    return a.type == cudaMemoryTypeUnregistered;
 }
 bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    if (bytes <= INLINE_COPY || host_pinned(src)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "copy to the device");
+    if (bytes <= INLINE_COPY || !pageable(src)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "copy to the device");
     if (!pinned_open()) return false;
     State &g = st();
     int i = 0;
@@ -92,7 +94,7 @@ bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     return true;
 }
 bool to_host(void *dst, const void *src, size_t bytes, cudaStream_t s, const volatile uint32_t *stop) {
-    if (host_pinned(dst)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "copy to the host");
+    if (!pageable(dst)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "copy to the host");
     if (!pinned_open()) return false;
     State &g = st();
     const size_t chunks = (bytes + RING_CHUNK - 1) / RING_CHUNK;
