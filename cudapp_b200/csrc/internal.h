@@ -77,9 +77,9 @@ uint64_t now_ns();
 // (3 MB to the host: 178 us, against 64 us of DMA). Up to 64 KB to the device the driver copies the bytes into its command buffer, which is
 // faster than either.
 constexpr size_t RESULT_BYTES = 32 * 1024;      // results up to this size are stored by the kernel itself into mapped host memory
-bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s);                      // src may be reused on return
-// pageable dst: complete on return; page-locked dst: complete once `s` is. stop (mapped host word, optional): when the work queued before this
-// call has set it, nothing is written to a pageable dst
+bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s);                      // pageable src: may be reused on return; any other: once `s` is past the copy
+// pageable dst: complete on return; any other: complete once `s` is. stop (mapped host word, optional): when the work queued before this
+// call has set it, nothing is written to dst
 bool to_host(void *dst, const void *src, size_t bytes, cudaStream_t s, const volatile uint32_t *stop = nullptr);
 void *result_area();                            // RESULT_BYTES of mapped page-locked memory and, behind it, a flag word; nullptr on failure
 inline volatile uint32_t *result_flag(void *area) { return reinterpret_cast<volatile uint32_t *>(static_cast<char *>(area) + RESULT_BYTES); }

@@ -94,7 +94,10 @@ bool to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     return true;
 }
 bool to_host(void *dst, const void *src, size_t bytes, cudaStream_t s, const volatile uint32_t *stop) {
-    if (!pageable(dst)) return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "copy to the host");
+    if (!pageable(dst)) {   // written by DMA, so the word is looked at first: 272 -> 277 us for a call with a [512, 1536] result
+        if (stop) { if (!cuda_ok(cudaStreamSynchronize(s), "copy to the host")) return false; if (*stop) return true; }
+        return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "copy to the host");
+    }
     if (!pinned_open()) return false;
     State &g = st();
     const size_t chunks = (bytes + RING_CHUNK - 1) / RING_CHUNK;

@@ -68,3 +68,23 @@ def test_layer_buffers(tensors, tokens, kind):
         assert np.array_equal(got.cpu().numpy().view(ref.dtype).reshape(ref.shape), ref)
     assert np.array_equal(ids, want[2]) and np.array_equal(w, want[3])
     api.lib.omega_gpu_moe_layer_free(layer)
+
+
+@pytest.mark.parametrize("kind", ["pageable", "page-locked"])
+@pytest.mark.parametrize("rows", [1, 16, 17, 300, 1100])
+def test_refused_result_is_left_alone(rows, kind):
+    """a word that equals the poison refuses the call, whatever the size of the result (16 rows: the last that the kernel stores itself), and y is as it was"""
+    E, n, k = 2, 512, 256
+    w8 = np.zeros((E, n, k), np.uint8); w8[1, 100, 0] = 0x38                   # one weight of 1
+    rc, t = api.fp8_tensor_upload(E, n, k, w8, np.full((E, n // 128, k // 128), 0x3f80, np.uint16)); assert rc == 0, api.last_error()
+    x = np.ones((rows, k), np.float32); x[rows // 2, 0] = -999.0
+    ids, tok = np.full(rows, 1, np.uint32), np.arange(rows, dtype=np.uint32)
+    y = in_memory(np.full((rows, n), 7, np.float32), kind)
+    rc = api.lib.omega_gpu_fp8gemm_f32(t, C.c_uint32(rows), api._p(ids), api._p(tok), api._p(x), C.c_uint32(rows), ptr(y), None)
+    assert rc == api.CHIP_FAIL and "poison" in api.last_error()
+    assert (y.numpy().view(np.float32) == 7).all()
+    x[rows // 2, 0] = 3                                                        # and the next call is served
+    rc = api.lib.omega_gpu_fp8gemm_f32(t, C.c_uint32(rows), api._p(ids), api._p(tok), api._p(x), C.c_uint32(rows), ptr(y), None); assert rc == 0, api.last_error()
+    want = np.zeros((rows, n), np.float32); want[:, 100] = x[:, 0]
+    assert np.array_equal(y.numpy().view(np.float32).reshape(rows, n), want)
+    api.fp8_tensor_free(t)
