@@ -183,8 +183,10 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? 5 : 3) fp8_rows_ker
 template <int LB, int R, int MT>
 static cudaError_t launch_one(const GemvArgs &a, dim3 grid, cudaStream_t s) {
     const size_t smem = (size_t)MT * (a.k < ROWS_CHUNK<MT> ? a.k : ROWS_CHUNK<MT>) * 4;
-    static const cudaError_t attr = cudaFuncSetAttribute(fp8_rows_kernel<LB, R, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MT * ROWS_CHUNK<MT> * 4));
-    if (attr != cudaSuccess) return attr;
+    if (smem > 40 * 1024) {   // near 48 KB with the static words; set on every call: it belongs to the device's context, and a failure must not outlive its call
+        const cudaError_t e = cudaFuncSetAttribute(fp8_rows_kernel<LB, R, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MT * ROWS_CHUNK<MT> * 4));
+        if (e != cudaSuccess) return e;
+    }
     return launch_chained(fp8_rows_kernel<LB, R, MT>, grid, dim3(32 * ROWS_WARPS), smem, s, a);
 }
 template <int R, int MT>
