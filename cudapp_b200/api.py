@@ -83,48 +83,91 @@ def _p(a):
 
 # ---------------------------------------------------------------- result arrays
 # Results of 64 KB or more live in page-locked memory: the device writes them by DMA, without the pass through a staging buffer that fresh pageable
-# pages need (a [512, 1536] f32 result: 64 us instead of 180). Page-locking costs milliseconds, so a block goes back to a free list when the last
-# array on it is gone; the list holds at most POOL_BYTES, and what does not fit is released.
-POOL_BYTES, POOL_MIN = 128 << 20, 64 << 10
-_pool, _pool_held, _pool_lock = {}, 0, threading.RLock()   # size -> free addresses; re-entrant: a collection inside the locked part may return a block
+# pages need (a [512, 1536] f32 result: a call of 285 us instead of 474). Page-locking itself costs milliseconds (1 MB 2.4, 4 MB 4.7, 32 MB 26), so blocks
+# are kept and go round. A program that drops its results needs one or two of a size; one that keeps them gets POOL_BLOCKS of each size and from then on
+# ordinary arrays, so that no call goes on page-locking. All blocks, in use or free, come to at most POOL_BYTES; where a new size would pass that, free blocks that
+# lay idle for POOL_IDLE results make room. Blocks are released there and never in a finaliser, which may run at any moment.
+POOL_MIN, POOL_BYTES, POOL_BLOCKS, POOL_IDLE = 64 << 10, 128 << 20, 4, 64
+
+
+class _Pool:
+    def __init__(self, alloc, release):
+        self.alloc, self.release = alloc, release
+        self.lock = threading.RLock()           # re-entrant: a collection inside the locked part may give a block back
+        self.free, self.blocks = {}, {}         # size -> (address, clock when it came back); size -> how many there are, in use or free
+        self.held = self.clock = 0
+
+    def take(self, size):
+        """the address of a block, or None where the result has to be an ordinary array"""
+        with self.lock:
+            self.clock += 1
+            if self.free.get(size):
+                return self.free[size].pop()[0]
+            if self.blocks.get(size, 0) >= POOL_BLOCKS:
+                return None
+            idle = self._idle(self.held + size - POOL_BYTES)
+            if idle is None:
+                return None
+            self.blocks[size] = self.blocks.get(size, 0) + 1
+            self.held += size
+        for address in idle:
+            self.release(address)
+        address = self.alloc(size)
+        if address is None:
+            with self.lock:
+                self.blocks[size] -= 1
+                self.held -= size
+        return address
+
+    def give(self, size, address):
+        with self.lock:
+            self.free.setdefault(size, []).append((address, self.clock))
+
+    def _idle(self, need):
+        """addresses of the longest idle blocks, taken out of the pool, that come to `need` bytes; None, and nothing taken, where there are not enough"""
+        out, found = [], 0
+        for since, size, address in sorted((since, size, address) for size, free in list(self.free.items()) for address, since in list(free)):
+            if found >= need or self.clock - since < POOL_IDLE:
+                break
+            out.append((since, size, address))
+            found += size
+        if found < need:
+            return None
+        for since, size, address in out:
+            self.free[size].remove((address, since))
+            self.blocks[size] -= 1
+            self.held -= size
+        return [address for _, _, address in out]
+
+
+def _host_alloc(size):
+    p = VP()
+    return p.value if lib.omega_gpu_host_alloc(C.c_uint64(size), C.byref(p)) == 0 else None
+
+
+_pool = _Pool(_host_alloc, lambda address: lib.omega_gpu_host_free(VP(address)))
 
 
 class _Block:
-    """one page-locked block as numpy's array interface sees it"""
-    __slots__ = ("addr", "size", "__array_interface__")
+    """one page-locked block as numpy's array interface sees it; it goes back when the last array on it is gone"""
+    __slots__ = ("pool", "size", "addr", "__array_interface__")
 
-    def __init__(self, addr, size, nbytes):
-        self.addr, self.size = addr, size
+    def __init__(self, pool, size, addr, nbytes):
+        self.pool, self.size, self.addr = pool, size, addr
         self.__array_interface__ = {"data": (addr, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
 
-    def __del__(self, free=lib.omega_gpu_host_free, lock=_pool_lock, pointer=C.c_void_p):
-        global _pool_held
-        with lock:
-            if _pool is not None and _pool_held + self.size <= POOL_BYTES:
-                _pool.setdefault(self.size, []).append(self.addr)
-                _pool_held += self.size
-                return
-        free(pointer(self.addr))
+    def __del__(self):
+        self.pool.give(self.size, self.addr)
 
 
 def _result(shape, dtype):
     """an uninitialised array for a result"""
-    global _pool_held
     nbytes = (shape if isinstance(shape, int) else math.prod(shape)) * np.dtype(dtype).itemsize
-    if nbytes < POOL_MIN:
-        return np.empty(shape, dtype)
-    size = 1 << (nbytes - 1).bit_length()
-    with _pool_lock:
-        free = _pool.get(size)
-        addr = free.pop() if free else None
-        if addr is not None:
-            _pool_held -= size
+    size = 1 << (nbytes - 1).bit_length() if nbytes >= POOL_MIN else 0
+    addr = _pool.take(size) if size else None
     if addr is None:
-        p = VP()
-        if lib.omega_gpu_host_alloc(C.c_uint64(size), C.byref(p)) != 0:
-            return np.empty(shape, dtype)
-        addr = p.value
-    return np.asarray(_Block(addr, size, nbytes)).view(dtype).reshape(shape)
+        return np.empty(shape, dtype)
+    return np.asarray(_Block(_pool, size, addr, nbytes)).view(dtype).reshape(shape)
 
 
 def last_error():

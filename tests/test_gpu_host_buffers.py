@@ -88,3 +88,21 @@ def test_refused_result_is_left_alone(rows, kind):
     want = np.zeros((rows, n), np.float32); want[:, 100] = x[:, 0]
     assert np.array_equal(y.numpy().view(np.float32).reshape(rows, n), want)
     api.fp8_tensor_free(t)
+
+
+def test_kept_results(tensors):
+    """results kept past what the binding page-locks: later ones lie in ordinary memory and all of them stay what they were"""
+    E, H, I, gu, _ = tensors
+    rng = np.random.default_rng(9)
+    ids = np.sort(rng.integers(0, E, 64)).astype(np.uint32); tok = np.arange(64, dtype=np.uint32)
+    x = [rng.normal(0, 1, (64, H)).astype(np.float32) for _ in range(12)]
+    kept = []
+    for v in x:                                                                # 128 KB each
+        rc, y = api.fp8gemm(gu, ids, tok, v); assert rc == 0, api.last_error()
+        kept.append(y)
+    before = api._pool.blocks[128 << 10]
+    assert before <= api.POOL_BLOCKS < len(kept) and api._pool.held <= api.POOL_BYTES
+    for v, y in zip(x, kept):
+        for r in (0, 31, 63):
+            rc, one = api.fp8gemm(gu, ids[r:r + 1], tok[:1], v[r:r + 1]); assert rc == 0, api.last_error()
+            assert np.array_equal(one[0].view(np.uint32), y[r].view(np.uint32))
