@@ -10,7 +10,6 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdlib.h>
-#include <vector>
 #include "internal.h"
 
 namespace b200 {
@@ -288,6 +287,14 @@ struct HostResult {
     }
 };
 
+// host bytes of one call; no exception may leave a C entry, so it is malloc's memory
+struct HostBytes {
+    char *p; size_t bytes;
+    explicit HostBytes(size_t n) : p((char *)malloc(n)), bytes(n) {}
+    ~HostBytes() { free(p); }
+    HostBytes(const HostBytes &) = delete;
+};
+
 // ids / x on the host, or tab / x on the device (dev form). y always a host buffer here.
 static int gemv_core(const OmegaGpuFp8Tensor *t, uint32_t groups, const uint32_t *ids, const float *x32, const uint16_t *x16,
                      uint32_t x_rows, float *y, OmegaGpuFp8Info *info, uint64_t dev_tab, uint64_t dev_x) {
@@ -305,10 +312,11 @@ static int gemv_core(const OmegaGpuFp8Tensor *t, uint32_t groups, const uint32_t
     if (dev_tab) a.tab = (const uint64_t *)(uintptr_t)dev_tab;
     else if (groups <= sizeof a.tab_inline / 16) for (uint32_t i = 0; i < groups; i++) (void)omega_gpu_fp8_tensor_entry(t, ids[i], &a.tab_inline[2 * i], &a.tab_inline[2 * i + 1]);
     else {
-        std::vector<uint64_t> ht((size_t)groups * 2);
+        HostBytes table((size_t)groups * 16);
+        uint64_t *ht = (uint64_t *)table.p, *tab = (uint64_t *)stage(0, table.bytes);
+        if (!ht) return OMEGA_GPU_FP8_BAD_ARGS;
         for (uint32_t i = 0; i < groups; i++) (void)omega_gpu_fp8_tensor_entry(t, ids[i], &ht[2 * i], &ht[2 * i + 1]);
-        uint64_t *tab = (uint64_t *)stage(0, ht.size() * 8);
-        if (!tab || !to_device(tab, ht.data(), ht.size() * 8, s)) return OMEGA_GPU_FP8_CHIP_FAIL;
+        if (!tab || !to_device(tab, ht, table.bytes, s)) return OMEGA_GPU_FP8_CHIP_FAIL;
         a.tab = tab;
     }
     if (!dev_x) {
@@ -349,23 +357,24 @@ static int gemm_core(const OmegaGpuFp8Tensor *t, uint32_t M, const uint32_t *ids
     if (!dev_open()) return OMEGA_GPU_FP8GEMM_CHIP_FAIL;
     const uint32_t n = t->n, k = t->k;
     const size_t xbytes = (size_t)x_rows * k * (x16 ? 2 : 4), sbytes = (size_t)segs * sizeof(Seg32);
-    std::vector<uint8_t> tables(sbytes + (size_t)M * 4);   // segment records, then the row table: one copy
-    Seg32 *hseg = (Seg32 *)tables.data();
-    memcpy(tables.data() + sbytes, trow, (size_t)M * 4);
+    HostBytes tables(sbytes + (size_t)M * 4);   // segment records, then the row table: one copy
+    if (!tables.p) return OMEGA_GPU_FP8GEMM_BAD_ARGS;
+    Seg32 *hseg = (Seg32 *)tables.p;
+    memcpy(tables.p + sbytes, trow, (size_t)M * 4);
     uint32_t sg = 0; uint64_t passes = 0, passes_max = 0;
     const uint32_t mt = gemm_rows_mt(k);
     for (uint32_t i = 0; i < M;) {
         uint32_t j = i; while (j < M && ids[j] == ids[i]) j++;
         (void)omega_gpu_fp8_tensor_entry(t, ids[i], &hseg[sg].w_va, &hseg[sg].s_va);
-        hseg[sg].row0 = i; hseg[sg].cnt = j - i;
+        hseg[sg].row0 = i; hseg[sg].cnt = j - i; hseg[sg].pad = 0;
         const uint32_t p = (j - i + mt - 1u) / mt; if (p > passes_max) passes_max = p;
         passes += p;
         sg++; i = j;
     }
     cudaStream_t s = g.stream;
-    char *dt = (char *)stage(0, tables.size()); void *xd = stage(1, xbytes);
+    char *dt = (char *)stage(0, tables.bytes); void *xd = stage(1, xbytes);
     HostResult r;
-    if (!dt || !xd || !to_device(dt, tables.data(), tables.size(), s) || !to_device(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, s) ||
+    if (!dt || !xd || !to_device(dt, tables.p, tables.bytes, s) || !to_device(xd, x32 ? (const void *)x32 : (const void *)x16, xbytes, s) ||
         !r.open((size_t)M * n, s)) return OMEGA_GPU_FP8GEMM_CHIP_FAIL;
     GemvArgs a = {};
     a.seg = (const Seg32 *)dt; a.x = xd; a.x_bf16 = x16 ? 1 : 0; a.x_rows = x_rows; a.xmap = (const uint32_t *)(dt + sbytes); a.ymap = nullptr;
