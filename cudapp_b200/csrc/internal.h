@@ -35,7 +35,7 @@ struct OmegaGpuW4Tensor {
     uint32_t n, k; uint8_t *w; uint16_t *s;   // s: fp16 scales (int4 format) or, viewed as bytes, E8M0 scales (MXFP4 format)
     uint32_t fmt;                              // 0: signed int4 + fp16 scale per 32; 1: MXFP4 = E2M1 + E8M0 scale per 32
     float *part; uint32_t *counters;   // scratch of the tensor-core kernel: K-quarter partial sums [4][16][n] f32 and one arrival counter per 128 output rows
-    uint32_t gtiles, gn;   // grouped form: most row tiles of a call, weight rows per expert; set by omega_gpu_w4_reserve_grouped
+    uint32_t gtiles, gn;   // omega_gpu_w4_gemm_grouped_async: most row tiles of a call, weight rows per expert; set by omega_gpu_w4_reserve_grouped
 };
 
 namespace b200 {
@@ -176,8 +176,9 @@ struct FfnLaunch {
     const unsigned long long *gate, *gate_base; const uint64_t *out_peers, *ret_counters; uint32_t rows_per_rank, ret_index;   // expert parallelism, as in MmaLaunch
     uint32_t wait_limit;
 };
-// grouped 4-bit GEMM over a plan's 16-row tiles (the tensor must have been given its shape by omega_gpu_w4_reserve_grouped)
-cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
+// grouped 4-bit GEMM over a plan's 16-row tiles: experts of n rows each (w4_grouped_ok), at most max_tiles tiles. The caller's own shape, nothing of the tensor's: layers may share it
+bool w4_grouped_ok(const OmegaGpuW4Tensor *t, uint32_t n);
+cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, uint32_t n, uint32_t max_tiles, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *x_bf16, uint16_t *y_bf16, float *y_f32, cudaStream_t s);
 bool ffn_shape_ok(uint32_t hidden, uint32_t inter);
 cudaError_t launch_ffn(const void *tm_gu, const void *tm_qx, const void *tm_dn, const void *tm_qa, uint32_t px, uint32_t pa, const FfnLaunch &m, cudaStream_t s, bool pdl);

@@ -31,15 +31,12 @@ int omega_gpu_moe_w4_layer_create(OmegaGpuW4Tensor *gate_up, OmegaGpuW4Tensor *d
     const uint32_t H = gate_up->k, I = down->k;
     if (gate_up->n / experts != 2u * I || down->n / experts != H) { set_error("w4 layer: gate|up must be experts x 2I rows of H columns and down experts x H rows of I columns"); return OMEGA_GPU_FP8_BAD_ARGS; }
     if (gate_up->fmt != down->fmt) { set_error("w4 layer: both tensors must have one weight format"); return OMEGA_GPU_FP8_BAD_ARGS; }
+    if (!w4_grouped_ok(gate_up, 2u * I) || !w4_grouped_ok(down, H)) return OMEGA_GPU_FP8_BAD_ARGS;
     OmegaGpuMoeW4Layer *L = (OmegaGpuMoeW4Layer *)calloc(1, sizeof *L);
     if (!L) return OMEGA_GPU_FP8_BAD_ARGS;
     L->gu = gate_up; L->dn = down; L->experts = experts; L->hidden = H; L->inter = I; L->topk = topk; L->max_tokens = max_tokens; L->norm_topk = norm_topk;
     const size_t T = max_tokens, R = T * topk;
     L->max_tiles = (uint32_t)(R / 16 + experts + 8);
-    // the shapes of the two grouped GEMMs (each call takes the library's lock itself)
-    int rc = omega_gpu_w4_reserve_grouped(gate_up, 2u * I, L->max_tiles);
-    if (rc == OMEGA_GPU_FP8_OK) rc = omega_gpu_w4_reserve_grouped(down, H, L->max_tiles);
-    if (rc != OMEGA_GPU_FP8_OK) { free(L); return rc; }
     Lock l;
     if (!dev_open()) { free(L); return OMEGA_GPU_FP8_CHIP_FAIL; }
     L->scratch_words = plan_scratch_words((uint32_t)R, experts);
@@ -53,6 +50,9 @@ int omega_gpu_moe_w4_layer_create(OmegaGpuW4Tensor *gate_up, OmegaGpuW4Tensor *d
     L->logits = (uint16_t *)(b + o_lg); L->x = (uint16_t *)(b + o_x); L->ids = (uint32_t *)(b + o_ids); L->wts = (float *)(b + o_wts); L->counts = (uint32_t *)(b + o_cnt);
     L->starts = (uint32_t *)(b + o_st); L->xmap = (uint32_t *)(b + o_xm); L->ymap = (uint32_t *)(b + o_ym); L->tiles = (uint32_t *)(b + o_tl); L->header = (uint32_t *)(b + o_hdr);
     L->scratch = (uint32_t *)(b + o_sc); L->gu32 = (float *)(b + o_gu); L->act16 = (uint16_t *)(b + o_act); L->dn32 = (float *)(b + o_dn); L->out32 = (float *)(b + o_o32); L->out16 = (uint16_t *)(b + o_o16);
+    // a tensor that has no shape for the grouped GEMM entry yet gets the layer's; the layer itself uses its own
+    if (!gate_up->gtiles) { gate_up->gtiles = L->max_tiles; gate_up->gn = 2u * I; }
+    if (!down->gtiles) { down->gtiles = L->max_tiles; down->gn = H; }
     *out = L;
     return OMEGA_GPU_FP8_OK;
 }
@@ -77,10 +77,10 @@ int omega_gpu_moe_w4_layer_async(OmegaGpuMoeW4Layer *L, uint32_t tokens, uint64_
     const bool ok = cuda_ok(launch_topk(tokens, E, K, L->norm_topk, (const uint16_t *)(uintptr_t)logits_va, L->ids, L->wts, s), "top-k launch") &&
                     cuda_ok(launch_plan(tokens, K, E, K, 16, L->ids, o, s, L->scratch, L->scratch_words), "plan launch") &&
                     // gate|up: sorted row p = x[xmap[p]] against its expert's 2I x H matrix, f32 in sorted order
-                    cuda_ok(launch_w4_grouped(L->gu, L->tiles, L->header, L->xmap, nullptr, (const uint16_t *)(uintptr_t)x_va, nullptr, L->gu32, s), "gate|up launch") &&
+                    cuda_ok(launch_w4_grouped(L->gu, 2u * I, L->max_tiles, L->tiles, L->header, L->xmap, nullptr, (const uint16_t *)(uintptr_t)x_va, nullptr, L->gu32, s), "gate|up launch") &&
                     cuda_ok(launch_swiglu(R, I, L->gu32, nullptr, s, L->act16), "swiglu launch") &&
                     // down: sorted row p against its expert's H x I matrix, result to row ymap[p] = token * K + slot
-                    cuda_ok(launch_w4_grouped(L->dn, L->tiles, L->header, nullptr, L->ymap, L->act16, nullptr, L->dn32, s), "down launch") &&
+                    cuda_ok(launch_w4_grouped(L->dn, H, L->max_tiles, L->tiles, L->header, nullptr, L->ymap, L->act16, nullptr, L->dn32, s), "down launch") &&
                     cuda_ok(launch_combine(tokens, K, H, L->wts, L->dn32, (float *)(uintptr_t)out_f32_va, (uint16_t *)(uintptr_t)out_bf16_va, s), "combine launch");
     L->launches = 6 + plan_launch_count(R, E, L->scratch, L->scratch_words, o) - 1u;
     return ok ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;

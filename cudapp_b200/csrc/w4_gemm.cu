@@ -467,15 +467,18 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
 }
 
 template <int FMT>
-static cudaError_t w4_grouped(const OmegaGpuW4Tensor *t, const W4Group &grp, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
+static cudaError_t w4_grouped(const OmegaGpuW4Tensor *t, uint32_t n, uint32_t max_tiles, const W4Group &grp, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often and were slower (before the decode by word, 64-token MXFP4 layer:
     // 279 us, 274 with 64 columns, 307 with 128; 64-token int4 layer of 32 experts, hidden 4096: 178, 188 and 203 us).
-    return w4_rows_start<FMT, 1, 2, 4, true>(t, 0, t->gn, t->gtiles, dx, d16, d32, grp, s);
+    return w4_rows_start<FMT, 1, 2, 4, true>(t, 0, n, max_tiles, dx, d16, d32, grp, s);
 }
-cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
+bool w4_grouped_ok(const OmegaGpuW4Tensor *t, uint32_t n) {
+    return n && n % 128u == 0 && t->n % n == 0 && (t->k == 768u || t->k == 1024u || t->k == 2048u || t->k == 4096u);
+}
+cudaError_t launch_w4_grouped(const OmegaGpuW4Tensor *t, uint32_t n, uint32_t max_tiles, const void *tiles, const uint32_t *header, const uint32_t *xmap, const uint32_t *ymap,
                               const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     const W4Group grp = {(const uint4 *)tiles, header, xmap, ymap};
-    return t->fmt == 2 ? w4_grouped<2>(t, grp, dx, d16, d32, s) : t->fmt ? w4_grouped<1>(t, grp, dx, d16, d32, s) : w4_grouped<0>(t, grp, dx, d16, d32, s);
+    return t->fmt == 2 ? w4_grouped<2>(t, n, max_tiles, grp, dx, d16, d32, s) : t->fmt ? w4_grouped<1>(t, n, max_tiles, grp, dx, d16, d32, s) : w4_grouped<0>(t, n, max_tiles, grp, dx, d16, d32, s);
 }
 
 }  // namespace b200
@@ -603,7 +606,7 @@ static cudaError_t w4_launch(const OmegaGpuW4Tensor *t, uint32_t m, const uint16
  * the rows to multiply come sorted by expert with a tile table of a routing plan made with tile_rows = 16 (omega_gpu_moe_plan_async: tiles {expert, first
  * row, rows}, header[2] = tiles). reserve sets the shape and the most tiles of a call; the async entry queues one launch and allocates nothing. */
 int omega_gpu_w4_reserve_grouped(OmegaGpuW4Tensor *t, uint32_t n_per_expert, uint32_t max_tiles) {
-    if (!t || !n_per_expert || !max_tiles || n_per_expert % 128u || t->n % n_per_expert || !(t->k == 768u || t->k == 1024u || t->k == 2048u || t->k == 4096u)) return OMEGA_GPU_FP8_BAD_ARGS;
+    if (!t || !max_tiles || !w4_grouped_ok(t, n_per_expert)) return OMEGA_GPU_FP8_BAD_ARGS;
     Lock l;
     if (!dev_open()) return OMEGA_GPU_FP8_CHIP_FAIL;
     t->gtiles = max_tiles; t->gn = n_per_expert;
@@ -614,7 +617,7 @@ int omega_gpu_w4_gemm_grouped_async(const OmegaGpuW4Tensor *t, uint64_t tiles_va
     if (!t || !tiles_va || !header_va || !x_bf16_va || (!y_bf16_va && !y_f32_va)) return OMEGA_GPU_FP8_BAD_ARGS;
     if (!t->gtiles) { set_error("w4 grouped gemm: call omega_gpu_w4_reserve_grouped first"); return OMEGA_GPU_FP8_BAD_ARGS; }
     if (!st().opened || st().latched) return OMEGA_GPU_FP8_CHIP_FAIL;
-    return cuda_ok(launch_w4_grouped(t, (const void *)(uintptr_t)tiles_va, (const uint32_t *)(uintptr_t)header_va, (const uint32_t *)(uintptr_t)xmap_va, (const uint32_t *)(uintptr_t)ymap_va,
+    return cuda_ok(launch_w4_grouped(t, t->gn, t->gtiles, (const void *)(uintptr_t)tiles_va, (const uint32_t *)(uintptr_t)header_va, (const uint32_t *)(uintptr_t)xmap_va, (const uint32_t *)(uintptr_t)ymap_va,
                                      (const uint16_t *)(uintptr_t)x_bf16_va, (uint16_t *)(uintptr_t)y_bf16_va, (float *)(uintptr_t)y_f32_va, (cudaStream_t)stream), "w4 grouped launch")
                ? OMEGA_GPU_FP8_OK : OMEGA_GPU_FP8_CHIP_FAIL;
 }

@@ -102,7 +102,7 @@ int omega_gpu_w4_gemm_grouped_async(const OmegaGpuW4Tensor *t, uint64_t tiles_va
 
 /* ---- one MoE layer with 4-bit expert weights (any of the three formats above; MXFP4 and NVFP4 are the reference's own 4-bit expert formats).
  * gate_up: experts x 2I rows of k = hidden (gate rows first, then up rows, per expert); down: experts x hidden rows of k = I; both uploaded with the
- * upload entry of their format, not owned by the layer and not usable by another layer at the same time (the layer reserves their grouped scratch).
+ * upload entry of their format, not owned by the layer; several layers may share them.
  * hidden and I in {768, 1024, 2048, 4096}. Steps: top-k of the bf16 logits (the reference's selection rule), routing plan, grouped gate|up, SiLU gate
  * rounded to bf16, grouped down, slot-order combine; 6 launches. */
 typedef struct OmegaGpuMoeW4Layer OmegaGpuMoeW4Layer;
