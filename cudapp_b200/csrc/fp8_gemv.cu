@@ -31,17 +31,21 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 template <int LB> __device__ __forceinline__ uint32_t xs_at(uint32_t q, uint32_t lane) { return q * 32u + (lane ^ (q * (LB == 16 ? 2u : LB == 8 ? 4u : 0u))); }
 
 // grid (ctas, groups or segments); 4 warps. A CTA puts MT activation rows of its segment into shared memory as f32, in the lanes' own column
-// order, and its warps then stream weight rows against them: R consecutive output rows per warp, the weights of the next two K steps in flight.
+// order, and its warps then stream weight rows against them: R consecutive output rows per warp, the weights of the next PF K steps in flight.
 // Bound by HBM when a segment has a few rows (64 tokens x 8 picks, [1536, 2048]: 400 MB), by the FP32 pipe from about four rows per expert on.
 // With one output row per warp and x read per row from global memory, as this kernel was, every product cost a load and a conversion beside its
 // FMA; four rows share them here, and fma.rn.f32x2 runs two rows' chains (each its own IEEE chain: the same bits) in one instruction slot.
 constexpr uint32_t ROWS_WARPS = 4;
 template <int MT> constexpr uint32_t ROWS_CHUNK = MT == 8 ? 2048u : 4096u;   // columns of x resident at a time: at most 64 KB, so that three CTAs share an SM
+constexpr uint32_t GEMV_CTAS = 8;   // of the one-row GEMV form on an SM: 64 registers a thread. Left to itself it took 74 to 80 and six fitted, so that grids up to eight ran in two waves
+// One row per warp: a lane has 64 bytes of weights in flight at every lane width. Four K steps whatever the width, as this was, are only 16 bytes where k is not a multiple of 256.
+// Both together, us with a cold L2, before -> now: 8 x [512, 3968] 38.9 -> 20.5, 5 x [768, 8192] 32.7 -> 23.3, 1 x [512, 8320] 42.9 -> 30.7, 3 x [1536, 4224] 43.0 -> 22.5. With four
+// rows per warp two steps stay: 32 bytes per row at every width took up to 84 registers, one CTA per SM fewer (8 x [1536, 8320] 47 -> 75 us).
 template <int LB, int R, int MT>
-__global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? 5 : 3) fp8_rows_kernel(const __grid_constant__ GemvArgs a) {
+__global__ void __launch_bounds__(32 * ROWS_WARPS, MT == 1 ? (R == 1 ? GEMV_CTAS : 5) : 3) fp8_rows_kernel(const __grid_constant__ GemvArgs a) {
     griddep_chain();
     constexpr uint32_t STEP = 32u * LB, CS = ROWS_CHUNK<MT> / STEP, Q = LB / 4, NT = 32u * ROWS_WARPS;
-    constexpr int PF = R == 1 ? 4 : 2, PAIRS = R > 1 ? R / 2 : 1;
+    constexpr int PF = R == 1 ? 64 / LB : 2, PAIRS = R > 1 ? R / 2 : 1;
     using WT = typename WVec<LB>::T;
     extern __shared__ float4 xs[];                 // [step of the chunk][MT][Q][32]
     __shared__ const uint8_t *s_row[MT];
@@ -196,11 +200,11 @@ static cudaError_t launch_lb(const GemvArgs &a, dim3 grid, cudaStream_t s) {
     return launch_one<4, R, MT>(a, grid, s);
 }
 
-// GEMV forms: one activation row per group. Four rows per warp once that leaves every SM two CTAs; below it one row per warp gives four times the
-// CTAs. A row's arithmetic does not depend on how rows are dealt to warps: same bits.
+// GEMV forms: one activation row per group. One row per warp while all of its CTAs are resident at once, else four rows per warp (a quarter of the CTAs,
+// each x value read once for four products). A row's arithmetic does not depend on how rows are dealt to warps: same bits.
 cudaError_t launch_gemv_grouped(const GemvArgs &a, uint32_t cta_budget, uint32_t *grid_x, uint32_t *warps, cudaStream_t s) {
     const uint32_t sms = st().sm_count ? st().sm_count : 148u;
-    const bool few = (uint64_t)(a.n / 16u) * a.groups_or_segs < 2u * sms && !cta_budget;
+    const bool few = (uint64_t)(a.n / ROWS_WARPS) * a.groups_or_segs <= GEMV_CTAS * sms && !cta_budget;
     uint32_t gx = few ? a.n / ROWS_WARPS : a.n / (4u * ROWS_WARPS);
     if (cta_budget && gx > cta_budget) gx = cta_budget;
     if (warps) *warps = ROWS_WARPS;

@@ -45,3 +45,27 @@ def test_grouped_gemv_result_sizes(groups):
     for y in kept + [pageable]:
         assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
     api.fp8_tensor_free(t)
+
+
+@pytest.mark.parametrize("k", [128, 640, 2304, 3968, 4096, 4224, 8192, 8320])
+def test_gemv_row_lengths(k):
+    """one row per warp (few groups) and four (many, or a CTA budget, where a CTA also makes several turns); x resident up to k = 4096 and by chunks past it;
+    all lane widths, fewer K steps than are prefetched, and remainders of them"""
+    rng = np.random.default_rng(k)
+    E, n = 3, 256
+    w8, sc = make_weights(rng, E, n, k)
+    rc, t = api.fp8_tensor_upload(E, n, k, w8, sc); assert rc == 0, api.last_error()
+    x = rng.normal(0, 1, (24, k)).astype(np.float32)
+    for groups, budget in ((1, 0), (2, 0), (18, 0), (19, 0), (24, 0), (2, 1), (2, 3), (24, 5)):
+        ids = rng.integers(0, E, groups).astype(np.uint32)
+        api.lib.omega_gpu_fp8_set_cta_budget(api.C.c_uint32(budget))
+        try:
+            rc, y = api.fp8_gemv_grouped_f32(t, ids, x[:groups]); assert rc == 0, api.last_error()
+        finally:
+            api.lib.omega_gpu_fp8_set_cta_budget(api.C.c_uint32(0))
+        for g, e in enumerate(ids):
+            assert np.array_equal(y[g].view(np.uint32), orc.gemv_emu(w8[e], sc[e], x[g]).view(np.uint32)), (groups, budget, g)
+    xb = orc.bf16_bits(x[0])
+    rc, y = api.fp8_gemv_bf16(t, 1, xb); assert rc == 0, api.last_error()
+    assert np.array_equal(y.view(np.uint32), orc.gemv_emu(w8[1], sc[1], orc.bf16_to_f32(xb)).view(np.uint32))
+    api.fp8_tensor_free(t)
