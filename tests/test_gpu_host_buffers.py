@@ -106,3 +106,18 @@ def test_kept_results(tensors):
         for r in (0, 31, 63):
             rc, one = api.fp8gemm(gu, ids[r:r + 1], tok[:1], v[r:r + 1]); assert rc == 0, api.last_error()
             assert np.array_equal(one[0].view(np.uint32), y[r].view(np.uint32))
+
+
+def test_result_that_takes_long(tensors):
+    """a small result is waited for in host memory for 2 ms at most and by the stream past that: a call behind work that fills the device for longer"""
+    import torch
+    E, H, I, gu, _ = tensors
+    x = np.random.default_rng(11).normal(0, 1, H).astype(np.float32)
+    rc, want = api.fp8_gemv_f32(gu, 3, x); assert rc == 0, api.last_error()
+    a, b = (torch.randn((8192, 8192), device="cuda") for _ in range(2))
+    torch.mm(a, b); torch.cuda.synchronize()
+    for _ in range(4):
+        torch.mm(a, b)                                                         # about 20 ms each in f32
+    rc, got = api.fp8_gemv_f32(gu, 3, x); assert rc == 0, api.last_error()
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    torch.cuda.synchronize()

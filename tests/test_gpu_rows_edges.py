@@ -1,6 +1,6 @@
-"""The exact row kernel and the host result paths where their shapes change: rows per pass (8, or 4 past k = 2048), x resident or staged by chunks
-(k = 4096), the three lane widths, and results around the size that is stored straight into host memory. Oracle: the reference kernels' own summation
-order, bit for bit."""
+"""The exact row kernel and the host result paths where their shapes change: rows per pass (8, or 4 past k = 2048), x resident (up to k = 4096) or staged by
+chunks past it, one turn or several per CTA, the three lane widths, and results around the size that is stored straight into host memory. Oracle: the reference
+kernels' own summation order, bit for bit."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,7 @@ def test_row_table_edges(n, k, bf16):
 
 @pytest.mark.parametrize("groups", [1, 8, 9, 63, 64, 65, 700])
 def test_grouped_gemv_result_sizes(groups):
-    """[groups, 128] f32 results: 64 groups are exactly the 32 KB that the kernel stores itself, 700 go through more than one staging chunk"""
+    """[groups, 128] f32 results: 64 groups are exactly the 32 KB that the kernel stores itself, 700 go through two staging chunks where the caller's array is pageable"""
     rng = np.random.default_rng(groups)
     E, n, k = 6, 128, 512
     w8, sc = make_weights(rng, E, n, k)
@@ -68,4 +68,25 @@ def test_gemv_row_lengths(k):
     xb = orc.bf16_bits(x[0])
     rc, y = api.fp8_gemv_bf16(t, 1, xb); assert rc == 0, api.last_error()
     assert np.array_equal(y.view(np.uint32), orc.gemv_emu(w8[1], sc[1], orc.bf16_to_f32(xb)).view(np.uint32))
+    api.fp8_tensor_free(t)
+
+
+@pytest.mark.parametrize("k", [640, 2048, 2304, 4224, 8192])
+def test_row_table_turns(k):
+    """96 segments of [512, k]: a CTA makes two turns over weight groups, so weights are fetched across turns and, past k = 4096, x is staged anew in the second;
+    segments of one, two and three passes among them"""
+    rng = np.random.default_rng(k)
+    E, n = 96, 512
+    w8 = rng.integers(0, 256, (E, n, k), dtype=np.uint8); w8[(w8 & 0x7f) == 0x7f] = 0
+    sc = rng.integers(0x3b00, 0x3c00, (E, n // 128, k // 128)).astype(np.uint16)
+    rc, t = api.fp8_tensor_upload(E, n, k, w8, sc); assert rc == 0, api.last_error()
+    counts = np.ones(E, np.int64); counts[5::16] = 4; counts[9::32] = 9; counts[20::48] = 17
+    ids = np.repeat(np.arange(E, dtype=np.uint32), counts)
+    xb = orc.bf16_bits(rng.normal(0, 1, (13, k)).astype(np.float32)); x = orc.bf16_to_f32(xb)
+    rows = rng.integers(0, 13, len(ids)).astype(np.uint32)
+    info = api.Fp8GemmInfo()
+    rc, y = api.fp8gemm(t, ids, rows, xb if k % 512 else x, info); assert rc == 0, api.last_error()
+    assert info.grid_x * 16 < n                                        # several turns
+    for i in range(len(ids)):
+        assert np.array_equal(y[i].view(np.uint32), orc.gemv_emu(w8[ids[i]], sc[ids[i]], x[rows[i]]).view(np.uint32)), (i, ids[i])
     api.fp8_tensor_free(t)
