@@ -20,7 +20,7 @@ struct FfnArgs {
     const uint4 *tiles; const uint32_t *header, *ymap;
     float *out;                                    // down results, row ymap[p], `hidden` floats each
     uint32_t hidden, inter, q_rows;
-    uint32_t *sched;                               // [0]: next down unit; [1 + tile]: gate|up units of that tile finished (zeroed by the plan kernel)
+    uint32_t *sched;                               // [0]: next down unit; [1 + tile]: gate|up units of that tile finished (zeroed by the kernel before: quantiser, gather or combine)
     uint32_t *err;
     // expert parallelism (null / 0 on one GPU): wait until peers have delivered header[0] input rows past *gate_base; down results go to the
     // owning rank's buffer (row y -> rank y / rows_per_rank) and each owner's counter [ret_index] is advanced once per delivered 256-feature slice

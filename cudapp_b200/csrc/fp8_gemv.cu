@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256) poison_scan_kernel(const float4 *__restri
 
 // A host call's result. Up to RESULT_BYTES the kernel stores it straight into mapped host memory, which was filled with poison before the launch: the
 // host takes each word as soon as it is no longer poison, and the call pays neither a fill kernel nor a copy nor a stream synchronisation (a single
-// [768, 2048] projection: 49 -> about 12 us per call). Larger results are poisoned, scanned and copied from device memory.
+// [768, 2048] projection called from Python, binding included: 49 -> 19 us). Larger results are poisoned, scanned and copied from device memory.
 struct HostResult {
     float *dev = nullptr; volatile float *mapped = nullptr; void *area = nullptr; size_t count; cudaStream_t s;
     bool open(size_t words, cudaStream_t stream) {

@@ -87,7 +87,8 @@ inline volatile uint32_t *result_flag(void *area) { return reinterpret_cast<vola
 struct Lock { Lock() { st().mu.lock(); } ~Lock() { st().mu.unlock(); } };
 
 // ---- programmatic dependent launch: the kernel may be set up while the one before it in the stream still runs, so that a chain of short kernels does not
-// pay a launch gap each. Every kernel launched this way begins with griddep_chain: it waits until the grids before it have completed and their
+// pay a launch gap each. Every kernel launched this way calls griddep_chain before it reads anything that earlier work wrote and before its own first write (the 4-bit kernel for
+// up to 16 rows requests its tensor's weights ahead of it, the others call it first): it waits until the grids before it have completed and their
 // writes are visible, and only then lets the next kernel start. So at any time only neighbours in the chain overlap, and a kernel that looks at
 // older results ahead of its own wait (the expert kernel reads the plan) finds them complete. Results of earlier kernels are read with plain loads
 // (no __restrict__ on const inputs, no __ldg): a load marked as invariant may be moved ahead of the wait.

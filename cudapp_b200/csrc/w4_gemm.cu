@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(512, GQ <= 16 ? 2 : 1) w4_mma_kernel(uint32_t 
 // quarter. A step is two scale groups of every quarter: rows of x (64 columns), weights (two 16-byte groups a row) and scales (4 bytes a row) come by
 // cp.async into one of two stages while the other is used. Two CTAs per SM (128 registers). The 16-byte chunks of a row of x are permuted by
 // bits 0 and 1 of the row, so that a quad's fragments of neighbouring rows fall on different banks.
-// Measured with a cold L2 against launches of 16 rows (int4 / MXFP4 / NVFP4): 300 x 4096 x 2048 169 / 171 / 205 -> 49 / 47 / 57 us, 17 x 4096 x 2048
-// 21.5 / 21.5 / 25.6 -> 14.3 us, 512 x 8192 x 4096 698 / 756 / 916 -> 199 / 215 / 262 us.
+// Measured with a cold L2 against launches of 16 rows (int4 / MXFP4 / NVFP4): 300 x 4096 x 2048 218 / 235 / 240 -> 49 / 47 / 58 us, 17 x 4096 x 2048
+// 25.6 / 25.6 / 28.6 -> 14.2 us, 512 x 8192 x 4096 855 / 921 / 1067 -> 199 / 214 / 262 us.
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, uint32_t bytes) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)); }
 __device__ __forceinline__ void cp4(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src)); }
 __device__ __forceinline__ uint32_t w4_chunk(uint32_t row, uint32_t c) { return c ^ (((row & 1u) << 2) | (row & 2u)); }
@@ -408,8 +408,10 @@ static cudaError_t w4_rows_start(const OmegaGpuW4Tensor *t, uint32_t m, uint32_t
 template <int FMT>
 static cudaError_t w4_rows(const OmegaGpuW4Tensor *t, uint32_t m, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
     // Few CTAs want small tiles, many want tall ones (a decoded weight is used more often); in between the number of waves decides. The cost of a tile is its
-    // MT x NT products, its decoding (NT) and a fixed part. Measured (int4, before the decode by word): 17 x 4096 x 2048 14.3 us at 2 x 2 and 26.6 at 4 x 4; 512 x 8192 x 4096 215 us at
-    // 4 x 4 and 268 at 2 x 2; 300 x 4096 x 2048 49 us at 5 x 4 (one wave, although some of its sums spill) and 55 at 4 x 4 (two waves).
+    // MT x NT products, its decoding (NT) and a fixed part. Measured, us with a cold L2, int4 / MXFP4 / NVFP4: 17 x 4096 x 2048 14 / 14 / 14 at 2 x 2, 25 / 25 / 29 at 4 x 4;
+    // 512 x 8192 x 4096 199 / 214 / 262 at 4 x 4, 262 / 272 / 330 at 2 x 2; 300 x 4096 x 2048 49 / 47 / 57 at 5 x 4 (one wave, although some of its sums spill), 53 / 55 / 66 at 4 x 4
+    // (two waves); 160 x 8192 x 1024 29 / 29 / 35 at 5 x 4, 31 / 33 / 39 at 4 x 4. Of 13 sizes (17 to 512 rows) in the three formats the rule took the fastest form or one within 9 %
+    // of it (400 x 3072 x 2048: 49 at 5 x 4, 45 at 3 x 4); 130 x 2048 x 768, 12 to 14 us in every form, is within 17 %.
     const uint32_t slots = 2u * (uint32_t)(st().sm_count ? st().sm_count : 148), tiles = (m + 15u) / 16u;
     uint32_t best = 0, cost = ~0u;
     for (uint32_t c = 0; c < 5; c++) {   // MT 2, 3, 4, 5 with NT = 4, then MT = 2 with NT = 2
@@ -468,8 +470,9 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_kernel(size_t blocks, cons
 
 template <int FMT>
 static cudaError_t w4_grouped(const OmegaGpuW4Tensor *t, uint32_t n, uint32_t max_tiles, const W4Group &grp, const uint16_t *dx, uint16_t *d16, float *d32, cudaStream_t s) {
-    // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often and were slower (before the decode by word, 64-token MXFP4 layer:
-    // 279 us, 274 with 64 columns, 307 with 128; 64-token int4 layer of 32 experts, hidden 4096: 178, 188 and 203 us).
+    // 32 columns a CTA: four CTAs per SM, and enough of them for one token's tiles. 64 and 128 columns re-read x less often, spill at 64 registers and are no faster. Measured, us, 32 / 64 / 128
+    // columns, 64-token layer of 128 experts, hidden 2048: int4 219 / 238 / 301, MXFP4 229 / 254 / 356, NVFP4 309 / 313 / 460; 512 tokens, 32 experts, hidden 4096: 830 / 890 / 1127,
+    // 900 / 995 / 1461, 1233 / 1219 / 1791.
     return w4_rows_start<FMT, 1, 2, 4, true>(t, 0, n, max_tiles, dx, d16, d32, grp, s);
 }
 bool w4_grouped_ok(const OmegaGpuW4Tensor *t, uint32_t n) {
